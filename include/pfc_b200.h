@@ -73,10 +73,11 @@ pfc_status  pfc_destroy(pfc_ctx* ctx);
  *                choice
  *   tiled        the register passes' field layout: 0 the reference layout, 1 kx tiles of
  *                8 columns (contiguous z and y column blocks); -1 the library's choice
- *   radix_order  the general (mixed-radix Stockham) passes: 0 radix 8 first, 1 radices 4
- *                and 2 only, 2 the odd radices first
+ *   radix_order  the general (mixed-radix) passes: 0 the fewest stages, 1 radices up to 5
+ *                (4 before 2), 2 the fewest stages with the odd radices first
  *   tile_shift   the general passes' lines per CTA halved this many times (0..4), for the
- *                x rows, the y columns, the z columns and the stepper's z pass
+ *                x rows, the y columns, the z columns and the stepper's z pass (2D fields:
+ *                its update pass along y)
  *   y_kernel     the register y pass between the kx-tiled layouts (ny = 512): 0 per-thread
  *                loads and stores, 1 the TMA unit moving whole tiles (bulk copies of the
  *                row-tiled blocks, tensor-map tile copies of the z-tiled pieces); -1 the

@@ -7,81 +7,127 @@
 #include <string>
 #include <vector>
 #include "bulk.cuh"
+#include "genpass.cuh"
 #include "pfc_ctx.h"
 
 using namespace pfc;
 
 namespace {
 
-// The radices of an n-point Stockham plan, in stage order.  order 0: radix 8 first, then
-// 4, 2, 3, 5 and the other primes up to kMaxOddRadix; 1: radices 4 and 2 only for the
-// power of two; 2: the odd radices first, then 8, 4, 2.
-bool factor_radices(int n, std::vector<int>& rs, int order = 0) {
+// The stages of an n-point plan of the general engine (genfft.cuh), in order.  order 0: the
+// fewest stages with radices up to `cap`, as equal as possible (the least sum), larger
+// radices first; 1: radices up to 5 (4 before 2); 2: as 0 with the odd radices first.  Primes
+// from 7 to kMaxOddRadix are stages of their own.  At least two stages, the last with a
+// hand-written DFT: a stage of radix 1 is appended where needed.
+bool factor_radices(int n, std::vector<int>& rs, int order, int cap) {
     rs.clear();
     if (n < 1) return false;
-    std::vector<int> pow2, odd;
-    if (order == 1) {
-        while (n % 4 == 0) { pow2.push_back(4); n /= 4; }
-    } else {
-        while (n % 8 == 0) { pow2.push_back(8); n /= 8; }
-        while (n % 4 == 0) { pow2.push_back(4); n /= 4; }
-    }
-    while (n % 2 == 0) { pow2.push_back(2); n /= 2; }
-    while (n % 3 == 0) { odd.push_back(3); n /= 3; }
-    while (n % 5 == 0) { odd.push_back(5); n /= 5; }
+    std::vector<int> primes;
     for (int p = 7; p <= kMaxOddRadix; p += 2) {
         bool prime = true;
         for (int d = 3; d * d <= p; d += 2) prime = prime && (p % d != 0);
         if (!prime) continue;
-        while (n % p == 0) { odd.push_back(p); n /= p; }
+        while (n % p == 0) { primes.push_back(p); n /= p; }
     }
-    if (order == 2) {
-        rs = odd;
-        rs.insert(rs.end(), pow2.begin(), pow2.end());
+    std::vector<int> best;
+    if (order == 1) {
+        for (int r : {4, 2, 3, 5})
+            while (n % r == 0) { best.push_back(r); n /= r; }
+        if (n != 1) return false;
     } else {
-        rs = pow2;
-        rs.insert(rs.end(), odd.begin(), odd.end());
+        static const int kRadix[] = {10, 9, 8, 6, 5, 4, 3, 2};
+        std::vector<int> cur;
+        int best_len = kMaxStages + 1, best_sum = 0;
+        // descending factorisations of n; the number of stages bounded by the best so far
+        auto search = [&](auto&& self, int rest, int from) -> void {
+            if (rest == 1) {
+                const int len = (int)cur.size();
+                int sum = 0;
+                for (int r : cur) sum += r;
+                if (len < best_len || (len == best_len && sum < best_sum)) {
+                    best = cur;
+                    best_len = len;
+                    best_sum = sum;
+                }
+                return;
+            }
+            if ((int)cur.size() >= best_len) return;
+            for (int i = from; i < (int)(sizeof(kRadix) / sizeof(kRadix[0])); ++i)
+                if (rest % kRadix[i] == 0 && kRadix[i] <= cap) {
+                    cur.push_back(kRadix[i]);
+                    self(self, rest / kRadix[i], i);
+                    cur.pop_back();
+                }
+        };
+        search(search, n, 0);
+        if (best_len > kMaxStages) return false;
+        if (order == 2) std::stable_partition(best.begin(), best.end(), [](int r) { return r % 2 != 0; });
     }
-    return n == 1 && (int)rs.size() <= kMaxStages;
+    rs = primes;
+    rs.insert(rs.end(), best.begin(), best.end());
+    if (best.empty() || rs.size() < 2) rs.push_back(1);
+    if (rs.size() < 2) rs.push_back(1);
+    return (int)rs.size() <= kMaxStages;
 }
 
-// Appends the Stockham twiddles of an n-point plan to tab (forward sign, FP64).
-bool make_plan(int n, LinePlan& p, std::vector<std::complex<double>>& tab, int order) {
+// Makes an n-point plan: appends its twiddles to tab (forward sign, FP64) and its index
+// tables to itab.
+bool make_plan(int n, GPlan& p, std::vector<std::complex<double>>& tab, std::vector<int>& itab, int order, int cap) {
     std::vector<int> rs;
-    if (!factor_radices(n, rs, order)) return false;
+    if (!factor_radices(n, rs, order, cap)) return false;
     std::memset(&p, 0, sizeof(p));
     p.n = n;
     p.nst = (int)rs.size();
+    p.rl = rs.back();
+    p.pad = p.rl % 2 == 0;
+    p.kstep = n / p.rl;
+    p.np = n + p.pad * p.kstep;
+    p.by_rl = make_fastdiv(p.rl);
     p.by_n = make_fastdiv(n);
-    int Ns = 1;
+    auto padded = [&](int i) { return i + p.pad * (i / p.rl); };
+    int M = n;
     for (int s = 0; s < p.nst; ++s) {
-        const int R = rs[s];
-        p.radix[s] = R;
-        p.ns[s] = Ns;
-        p.twoff[s] = (int)tab.size();
-        for (int jj = 0; jj < Ns; ++jj)
-            for (int r = 1; r < R; ++r) {
-                const long long num = ((long long)r * jj) % ((long long)Ns * R);
-                const double ang = -2.0 * M_PI * (double)num / (double)(Ns * R);
+        GStage& g = p.st[s];
+        g.R = rs[s];
+        g.m = M / g.R;
+        g.nb = n / g.R;
+        p.nbmax = std::max(p.nbmax, g.nb);
+        g.ms = s == p.nst - 1 ? 1 : padded(g.m);
+        g.Ms = padded(M);
+        g.by_m = make_fastdiv(g.m);
+        g.by_nb = make_fastdiv(g.nb);
+        g.tw = (int)tab.size();
+        for (int r = 1; r < g.R; ++r)
+            for (int j = 0; j < g.m; ++j) {
+                const double ang = -2.0 * M_PI * (double)(((long long)r * j) % M) / (double)M;
                 tab.emplace_back(std::cos(ang), std::sin(ang));
             }
-        p.rtoff[s] = (int)tab.size();
-        p.by_m[s] = make_fastdiv(n / R);
-        p.by_ns[s] = make_fastdiv(Ns);
-        if (R > 5)
-            for (int q = 0; q < R; ++q) {
-                const double ang = -2.0 * M_PI * (double)q / (double)R;
+        g.rt = (int)tab.size();
+        if (g.R >= 7 && g.R % 2 && g.R != 9)
+            for (int q = 0; q < g.R; ++q) {
+                const double ang = -2.0 * M_PI * (double)q / (double)g.R;
                 tab.emplace_back(std::cos(ang), std::sin(ang));
             }
-        Ns *= R;
+        M = g.m;
     }
+    // frequency of position q: digits of q by the stages, reversed
+    std::vector<int> freq(n);
+    for (int q = 0; q < n; ++q) {
+        int rest = q, k = 0, w = 1;
+        for (int s = 0; s < p.nst; ++s) {
+            const int d = rest / p.st[s].m;
+            rest -= d * p.st[s].m;
+            k += d * w;
+            w *= p.st[s].R;
+        }
+        freq[q] = k;
+    }
+    p.rev = (int)itab.size();
+    for (int b = 0; b < p.kstep; ++b) itab.push_back(freq[b * p.rl]);
+    p.pos = (int)itab.size();
+    itab.resize(itab.size() + n);
+    for (int q = 0; q < n; ++q) itab[p.pos + freq[q]] = padded(q);
     return true;
-}
-
-int pow2_floor(size_t v, int cap) {
-    int t = 1;
-    while (t * 2 <= cap && (size_t)(t * 2) <= v) t *= 2;
-    return t;
 }
 
 pfc_status fail(pfc_ctx* c, pfc_status s, const std::string& msg) {
@@ -114,7 +160,7 @@ void free_ctx(pfc_ctx* c) {
     if (c->side_fork) cudaEventDestroy(c->side_fork);
     if (c->side_join) cudaEventDestroy(c->side_join);
     if (c->side_stream) cudaStreamDestroy(c->side_stream);
-    void* ptrs[] = {c->tw,          c->work,         c->work2,        c->red,       c->k0,
+    void* ptrs[] = {c->tw,          c->gtw,          c->fft_tab,      c->work,         c->work2,        c->red,       c->k0,
                     c->flag,        c->peak_counts,  c->peak_offsets, c->bond_scratch, c->bond_pairs,
                     c->peak_mask};
     for (void* p : ptrs)
@@ -214,6 +260,7 @@ constexpr int kLayZ = 1, kLayRow = 2;
 // work2 (the psi^ buffer then holds the row-tiled field of the x pass), else in place of
 // psi^.
 void* carried_A(pfc_ctx* ctx, void* kpsi) {
+    if (ctx->nz == 1) return ctx->work;
     if (ctx->tiled) return ctx->z_carry ? ctx->work : ctx->work2;
     return ctx->z_carry ? ctx->work2 : kpsi;
 }
@@ -244,9 +291,13 @@ cudaError_t step_entry(pfc_ctx* ctx, void* kpsi) {
             if (!e) e = launch_zfft(ctx, 1, kpsi, ctx->work, 1.0 / ctx->nz, kLayZ << 2, 0, -1, ctx->work2);
             return e;
         });
-    return traced(ctx, 0, ctx->nz > 1 ? 2 : 1, [&] {
+    if (ctx->nz == 1)  // 2D: A = IFFT_y(psi^)/ny, psi^ carried in its buffer
+        return traced(ctx, 0, 1, [&] { return launch_cols(ctx, 1, 1, kpsi, ctx->work, 1.0 / ctx->ny); });
+    if (ctx->z_carry && !ctx->fused_z)  // the inverse transform of the z pass itself; psi^ keeps its k = 0 mode
+        return traced(ctx, 0, 1, [&] { return launch_cols(ctx, 2, 1, kpsi, ctx->work2, 1.0 / ctx->nz); });
+    return traced(ctx, 0, 2, [&] {
         cudaError_t e = launch_k0_save(ctx, kpsi);
-        if (e || ctx->nz == 1) return e;
+        if (e) return e;
         return zcols(ctx, 1, kpsi, carried_A(ctx, kpsi), 1.0 / ctx->nz, ctx->tiled ? kLayZ << 2 : 0);
     });
 }
@@ -255,10 +306,9 @@ cudaError_t step_entry(pfc_ctx* ctx, void* kpsi) {
 // (nothing to do when psi^ is carried)
 cudaError_t step_exit(pfc_ctx* ctx, void* kpsi) {
     if (ctx->tiled && ctx->z_carry) return traced(ctx, 0, 1, [&] { return launch_relayout(ctx, ctx->work2, kpsi, 0); });
-    if (ctx->z_carry) return cudaSuccess;
-    return traced(ctx, 0, ctx->nz > 1 ? 2 : 1, [&] {
-        cudaError_t e = ctx->nz > 1 ? zcols(ctx, -1, carried_A(ctx, kpsi), kpsi, 1.0, ctx->tiled ? kLayZ : 0)
-                                    : cudaSuccess;
+    if (ctx->z_carry || ctx->nz == 1) return cudaSuccess;
+    return traced(ctx, 0, 2, [&] {
+        cudaError_t e = zcols(ctx, -1, carried_A(ctx, kpsi), kpsi, 1.0, ctx->tiled ? kLayZ : 0);
         if (e) return e;
         return launch_k0_restore(ctx, kpsi);
     });
@@ -272,6 +322,11 @@ cudaError_t step_exit(pfc_ctx* ctx, void* kpsi) {
 cudaError_t step_xy(pfc_ctx* ctx, void* kpsi, const pfc_step_params* p, bool last) {
     const void* A = carried_A(ctx, kpsi);
     void* B = ctx->work;
+    if (ctx->nz == 1)  // 2D: the rows of A in place (the y transforms are the update pass's)
+        return traced(ctx, 1, 1, [&] {
+            if (ctx->xy_mode == 2) return launch_xpass(ctx, B, nullptr, 1.0 / ctx->nx, p->C, p->mu, 1);
+            return launch_rows_nonlin(ctx, B, 1.0 / ctx->nx, p->C, p->mu);
+        });
     const double mul = 1.0 / ((double)ctx->nx * (double)ctx->ny);
     if (ctx->tiled) {
         void* R = row_field(ctx, kpsi);
@@ -286,13 +341,11 @@ cudaError_t step_xy(pfc_ctx* ctx, void* kpsi, const pfc_step_params* p, bool las
             ctx, [&] { return launch_ypass(ctx, 1, A, B, 1.0, ctx->nz); },
             [&] { return launch_xpass(ctx, B, nullptr, mul, p->C, p->mu, ctx->nz); },
             [&] { return launch_ypass(ctx, -1, B, B, 1.0, ctx->nz); });
-    return traced(ctx, 1, ctx->ny > 1 ? 3 : 1, [&] {
-        cudaError_t e;
-        if (ctx->ny > 1) e = launch_cols(ctx, 1, 1, A, B, 1.0);
-        else e = cudaMemcpyAsync(B, A, ctx->state_bytes * ctx->batch, cudaMemcpyDeviceToDevice, ctx->stream);
+    return traced(ctx, 1, 3, [&] {
+        cudaError_t e = launch_cols(ctx, 1, 1, A, B, 1.0);
         if (e) return e;
-        if ((e = launch_rows_nonlin(ctx, B, nullptr, mul, p->C, p->mu))) return e;
-        return ctx->ny > 1 ? launch_cols(ctx, 1, -1, B, B, 1.0) : cudaSuccess;
+        if ((e = launch_rows_nonlin(ctx, B, mul, p->C, p->mu))) return e;
+        return launch_cols(ctx, 1, -1, B, B, 1.0);
     });
 }
 
@@ -302,6 +355,8 @@ cudaError_t step_xy(pfc_ctx* ctx, void* kpsi, const pfc_step_params* p, bool las
 // and the last step writes psi^' over B (standard layout, in place).
 cudaError_t step_z(pfc_ctx* ctx, void* kpsi, const ZPropArgs& za) {
     void* B = ctx->work;
+    if (ctx->nz == 1)  // 2D: along y, psi^' in its buffer and A' over B
+        return traced(ctx, 2, 1, [&] { return launch_zprop_carry(ctx, kpsi, B, B, za); });
     if (ctx->tiled && ctx->z_carry)
         return traced(ctx, 2, 1, [&] {
             return launch_zcarry_tiled(ctx, ctx->work2, ctx->work, za.final_step ? kpsi : ctx->work2,
@@ -467,15 +522,26 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     std::vector<std::complex<double>> tab;
     const bool even = (c->nx % 2) == 0;
     const int lx = even ? c->nx / 2 : c->nx;
-    if (!make_plan(lx, c->px.plan, tab, o.radix_order) || !make_plan(c->ny, c->py.plan, tab, o.radix_order) ||
-        !make_plan(c->nz, c->pz.plan, tab, o.radix_order)) {
+    std::vector<std::complex<double>> gtab;
+    std::vector<int> itab;
+    // Radices of the general passes by field size.  Small fields leave most of the GPU idle and
+    // pay for every instruction fetched, so small radices (more threads, less code) win: 256^2
+    // FP64 x pass 5.7 us at radices up to 6, 7.0 at 8 and 10; 600 x 500 FP32 8.0 at 8, 10.0 at
+    // 10; from about a million modes fewer stages win (160 x 150 x 160 FP32 x pass 14.7 at 10,
+    // 17.4 at 8).
+    const int cap = c->n_cmpl < 100000 ? 6 : c->n_cmpl < 1000000 ? 8 : 10;
+    if (!make_plan(lx, c->px.plan, gtab, itab, o.radix_order, cap) ||
+        !make_plan(c->ny, c->py.plan, gtab, itab, o.radix_order, cap) ||
+        !make_plan(c->nz, c->pz.plan, gtab, itab, o.radix_order, cap)) {
         free_ctx(c);
         return PFC_ERR_UNSUPPORTED;
     }
-    c->post_off = (int)tab.size();
+    c->pzprop.plan = c->pz2.plan = c->pz.plan;
+    c->py2.plan = c->py.plan;
+    c->post_off = (int)gtab.size();
     for (int k = 0; k <= c->nx / 2; ++k) {
         const double ang = -2.0 * M_PI * (double)k / (double)c->nx;
-        tab.emplace_back(std::cos(ang), std::sin(ang));
+        gtab.emplace_back(std::cos(ang), std::sin(ang));
     }
     auto roots = [&](int n, int count) {
         for (int m = 0; m < count; ++m) {
@@ -573,29 +639,48 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
             cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
         cudaGetLastError();
     }
-    // tiles: two ping-pong buffers of `tile` lines per CTA, halved tile_shift times; a pass
-    // with few lines takes smaller tiles, so that it still has two CTAs per SM
-    auto shifted = [](int t, int sh) { return std::max(1, t >> sh); };
-    auto fit = [&](int t, int64_t lines) {
-        while (t > 1 && (lines + t - 1) / t < 2 * (int64_t)c->num_sms) t >>= 1;
-        return t;
+    // lengths whose lines (two of them, padded one element per 32) do not fit a CTA's shared
+    // memory are refused
+    {
+        auto line = [&](int n, int lines) { return (size_t)lines * ((n + (n >> 5) + 1) | 1) * csz; };
+        if (line(lx, 2) > kMaxDynSmem || line(c->ny, 2) > kMaxDynSmem || line(c->nz, 4) > kMaxDynSmem) {
+            free_ctx(c);
+            return PFC_ERR_UNSUPPORTED;
+        }
+    }
+    // Lines per CTA of the general passes.  Columns: 128-byte segments (8 elements of 16 bytes:
+    // 16 FP32 or 8 FP64 columns), halved down to the 32-byte sectors of L2 while the tile's
+    // shared memory would leave fewer than three CTAs per SM, or the pass fewer than two CTAs
+    // per SM; then tile_shift times.  Threads: one butterfly each in the stage with the most, up
+    // to 256 (FP64: 128, for more CTAs per SM, unless the pass has too few CTAs for that).
+    // Rows: as many as fill those threads.
+    const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
+    const int many = c->dtype == PFC_F64 ? 128 : 256;
+    auto columns = [&](AxisPlan& ap, int64_t planes, int fields, int shift) {
+        const size_t line = (size_t)ap.plan.np * 16 * fields;
+        int lg = 3;
+        auto ctas = [&] { return ((c->nxh + (W << lg) - 1) / (W << lg)) * planes; };
+        while (lg > 1 && ((line << lg) > 72 * 1024 || ctas() < 2 * (int64_t)c->num_sms)) --lg;
+        while (lg > 0 && (line << lg) > kMaxDynSmem) --lg;
+        lg = std::max(0, lg - shift);
+        ap.lg = lg;
+        const int most = ctas() < 4 * (int64_t)c->num_sms ? kGenThreads : many;
+        ap.threads = std::min(most, std::max(32, ((ap.plan.nbmax * fields << lg) + 31) & ~31));
+        ap.smem = ((size_t)ap.plan.np * 16) << lg;
     };
-    const int64_t nyz = (int64_t)c->ny * c->nz;
-    c->px.tile = shifted(fit(pow2_floor((64 * 1024) / (2 * (size_t)lx * csz), 16), nyz), o.tile_shift[0]);
-    c->px.smem = 2 * (size_t)c->px.tile * line_stride(lx) * csz;
-    c->py.tile = shifted(fit(pow2_floor((64 * 1024) / (2 * (size_t)c->ny * csz), 16), (int64_t)c->nxh * c->nz),
-                         o.tile_shift[1]);
-    c->py.smem = 2 * (size_t)c->py.tile * line_stride(c->ny) * csz;
-    c->pz.tile = shifted(fit(pow2_floor((64 * 1024) / (2 * (size_t)c->nz * csz), 16), (int64_t)c->nxh * c->ny),
-                         o.tile_shift[2]);
-    c->pz.smem = 2 * (size_t)c->pz.tile * line_stride(c->nz) * csz;
-    c->pzprop.tile = shifted(fit(pow2_floor((96 * 1024) / (4 * (size_t)c->nz * csz), 8), (int64_t)c->nxh * c->ny),
-                             o.tile_shift[3]);
-    c->pzprop.smem = 4 * (size_t)c->pzprop.tile * line_stride(c->nz) * csz;
-    if (c->px.smem > kMaxDynSmem || c->py.smem > kMaxDynSmem || c->pz.smem > kMaxDynSmem ||
-        c->pzprop.smem > kMaxDynSmem) {
-        free_ctx(c);
-        return PFC_ERR_UNSUPPORTED;
+    columns(c->py, c->nz, 1, o.tile_shift[1]);
+    columns(c->pz, c->ny, 1, o.tile_shift[2]);
+    columns(c->pzprop, c->ny, 1, o.tile_shift[3]);
+    columns(c->pz2, c->ny, 2, o.tile_shift[3]);
+    columns(c->py2, 1, 1, o.tile_shift[3]);
+    {
+        AxisPlan& ap = c->px;
+        const int64_t nrows = (int64_t)c->ny * c->nz;
+        int lines = std::max(1, many / ap.plan.nbmax);
+        while (lines > 1 && (nrows + lines * W - 1) / (lines * W) < 2 * (int64_t)c->num_sms) lines >>= 1;
+        ap.lines = std::max(1, lines >> o.tile_shift[0]);
+        ap.threads = std::min(kGenThreads, std::max(32, (ap.lines * ap.plan.nbmax + 31) & ~31));
+        ap.smem = (size_t)ap.lines * ap.plan.np * 16;
     }
     c->n_peak_blocks = peak_chunks(c->nx, c->ny, c->nz);
     // bond order starts with room for 4096 atoms and 64 neighbours each; pfc_bond_order
@@ -608,7 +693,9 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     auto alloc = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     };
-    alloc(&c->tw, tab.size() * csz);
+    alloc(&c->tw, std::max<size_t>(1, tab.size()) * csz);
+    alloc(&c->gtw, gtab.size() * 16);
+    alloc((void**)&c->fft_tab, itab.size() * sizeof(int));
     alloc(&c->work, c->state_bytes);
     alloc(&c->work2, c->state_bytes);
     alloc((void**)&c->red, sizeof(double) * (kRedBlocks + 8));
@@ -626,11 +713,19 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     }
     if (c->dtype == PFC_F64) {
         e = cudaMemcpy(c->tw, tab.data(), tab.size() * csz, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(c->gtw, gtab.data(), gtab.size() * 16, cudaMemcpyHostToDevice);
     } else {
+        std::vector<float4> g32(gtab.size());  // each factor twice: {re, re, im, im}
+        for (size_t i = 0; i < gtab.size(); ++i) {
+            const float re = (float)gtab[i].real(), im = (float)gtab[i].imag();
+            g32[i] = make_float4(re, re, im, im);
+        }
+        e = cudaMemcpy(c->gtw, g32.data(), gtab.size() * 16, cudaMemcpyHostToDevice);
         std::vector<float2> t32(tab.size());
         for (size_t i = 0; i < tab.size(); ++i) t32[i] = make_float2((float)tab[i].real(), (float)tab[i].imag());
-        e = cudaMemcpy(c->tw, t32.data(), tab.size() * csz, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(c->tw, t32.data(), tab.size() * csz, cudaMemcpyHostToDevice);
     }
+    if (e == cudaSuccess) e = cudaMemcpy(c->fft_tab, itab.data(), itab.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(c->flag, 0, sizeof(int) * 4);
     if (e == cudaSuccess) e = set_fft_attributes(c);
     if (e == cudaSuccess && c->fused_z) e = set_zcol_attributes(c);
@@ -996,7 +1091,7 @@ pfc_status pfc_slab_xy(pfc_ctx* ctx, const void* A, void* B, double C, double mu
     } else {
         if (ctx->ny > 1) PFC_CUDA(launch_cols(ctx, 1, 1, A, B, 1.0), "pfc_slab_xy y");
         else PFC_CUDA(cudaMemcpyAsync(B, A, ctx->state_bytes, cudaMemcpyDeviceToDevice, ctx->stream), "pfc_slab_xy");
-        PFC_CUDA(launch_rows_nonlin(ctx, B, nullptr, mul, C, mu), "pfc_slab_xy x");
+        PFC_CUDA(launch_rows_nonlin(ctx, B, mul, C, mu), "pfc_slab_xy x");
         if (ctx->ny > 1) PFC_CUDA(launch_cols(ctx, 1, -1, B, B, 1.0), "pfc_slab_xy y");
     }
     ctx->launches += 3;
@@ -1337,12 +1432,15 @@ pfc_status pfc_ensemble_run(pfc_ensemble* e, int nsteps, void* stream) {
             pfc_ctx* c = e->ctx[i];
             c->stream = st;
             ce = step_entry(c, e->kpsi[i]);
-            // A: in the psi^ buffer, or in work for the tiled psi^-carrying schedule
-            const bool awork = c->tiled && c->z_carry;
+            // A: in the psi^ buffer, or in work for the tiled psi^-carrying schedule; 2D: psi^ in its
+            // buffer, A in work, nothing in work2
+            const bool flat = c->nz == 1, awork = c->tiled && c->z_carry;
             if (!ce)
                 ce = cudaMemcpyAsync((char*)(awork ? k.cc->work : k.state) + q * S, awork ? c->work : e->kpsi[i], S,
                                      cudaMemcpyDeviceToDevice, st);
-            if (!ce) ce = cudaMemcpyAsync((char*)k.cc->work2 + q * S, c->work2, S, cudaMemcpyDeviceToDevice, st);
+            if (!ce)
+                ce = cudaMemcpyAsync((char*)(flat ? k.cc->work : k.cc->work2) + q * S, flat ? c->work : c->work2, S,
+                                     cudaMemcpyDeviceToDevice, st);
             if (!ce) ce = cudaMemcpyAsync(k.cc->k0 + q, c->k0, sizeof(double2), cudaMemcpyDeviceToDevice, st);
             if (!ce) ce = launch_counter(st, k.ctr + q, e->p[i].counter, 1);
         }
@@ -1358,7 +1456,8 @@ pfc_status pfc_ensemble_run(pfc_ensemble* e, int nsteps, void* stream) {
             const bool awork = c->tiled && c->z_carry;  // (psi^ is in work2 then: A is not needed)
             ce = awork ? cudaSuccess
                        : cudaMemcpyAsync(e->kpsi[i], (char*)k.state + q * S, S, cudaMemcpyDeviceToDevice, st);
-            if (!ce) ce = cudaMemcpyAsync(c->work2, (char*)k.cc->work2 + q * S, S, cudaMemcpyDeviceToDevice, st);
+            if (!ce && c->nz > 1)
+                ce = cudaMemcpyAsync(c->work2, (char*)k.cc->work2 + q * S, S, cudaMemcpyDeviceToDevice, st);
             if (!ce) ce = step_exit(c, e->kpsi[i]);
         }
     }

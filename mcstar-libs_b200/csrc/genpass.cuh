@@ -1,0 +1,49 @@
+// The general-length passes over the reference layout (x fastest; half spectrum of nx/2+1
+// complex per row): whole lines of a tile in shared memory, transformed by the engine of
+// genfft.cuh.  They serve the reference-shaped primitives (R2C, C2R) and the stepper wherever
+// a length has no register kernel, in FP32 and FP64.  kern_gen*.cu instantiate them.
+#pragma once
+#include "genfft.cuh"
+#include "pfc_ctx.h"
+
+namespace pfc {
+
+template <typename T> cudaError_t gen_attrs();
+template <typename T> cudaError_t gen_cols(const pfc_ctx* c, int axis, int dir, const void* in, void* out, double scale);
+enum { kR2C = 0, kC2R = 1, kNonlin = 2 };
+template <typename T>
+cudaError_t gen_rows(const pfc_ctx* c, int mode, const void* in, void* out, double mul, double C, double mu);
+template <typename T> cudaError_t gen_zattrs();
+template <typename T>
+cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs& a, void* anext, bool carry, bool flat);
+
+// Register budget of the general passes: FP32 64 (four CTAs of 256 threads per SM), FP64 80
+// (six of 128; a radix-10 butterfly holds 40 of them, and its FP64 arithmetic needs more
+// temporaries).  They are latency-bound: at 128 registers and radices up to 16 the passes of
+// 240 x 200 x 180 FP32 took 0.025 / 0.049 / 0.088 ms (y, x, z) against 0.021 / 0.044 / 0.060.
+template <typename T> constexpr int kGenCtas = sizeof(T) == 8 ? 3 : 4;
+constexpr int kGenThreads = 256;
+
+// The columns of a CTA: 2^lg elements of one column (FP64) or of two columns 2^lg apart (FP32;
+// consecutive threads then move consecutive columns of either half), from column i0 of ni.
+template <typename T> struct ColTile {
+    int i0, n, second;
+    __device__ __forceinline__ ColTile(int lg, int ni, int col0 = 0) {
+        i0 = col0 + blockIdx.x * (Elem<T>::lines << lg);
+        n = ni - i0;
+        second = 1 << lg;
+    }
+    __device__ __forceinline__ bool ok(int i, int half) const { return i + half * second < n; }
+    // the elements of position i at g (column i0 + i), step apart
+    __device__ __forceinline__ auto get(const cx<T>* g, int i, int64_t step) const {
+        const bool ok0 = ok(i, 0), ok1 = ok(i, 1);
+        const cx<T>* h = g + second;
+        return [=](int r) {
+            const cx<T> z = mkc<T>(T(0), T(0));
+            const cx<T> a = ok0 ? g[r * step] : z;
+            return Elem<T>::pack(a, Elem<T>::lines > 1 && ok1 ? h[r * step] : z);
+        };
+    }
+};
+
+}  // namespace pfc

@@ -1,0 +1,245 @@
+// The general column and row passes (genpass.cuh): kernels and launchers, instantiated per
+// precision by kern_gen32.cu and kern_gen64.cu.
+#pragma once
+#include "genpass.cuh"
+
+namespace pfc {
+namespace {
+
+// ---------------------------------------------------------------------------------
+// complex FFT along a strided axis: element (line o, inner i, position k) at
+// base + o*os + i + k*es.  A CTA owns 2^lg elements (FP64: lines,
+// FP32: pairs of lines) of consecutive inner lines of one o.  Forward
+// transforms run down from natural order, inverse ones up to it: the inverse is then, bit
+// for bit, the one of the stepper's z pass (k_zprop).
+// ---------------------------------------------------------------------------------
+template <typename T, int DIR>
+__global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
+    k_cols(const cx<T>* in, cx<T>* out, int ni, int64_t es, int64_t os, const __grid_constant__ GPlan p,
+           const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, double scale, int64_t ms) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
+    const ColLines lay{lg};
+    const ColTile<T> tile{lg, ni};
+    const int64_t base = (int64_t)blockIdx.y * os + tile.i0 + blockIdx.z * ms;  // grid z: fields of a batch
+    in += base;
+    out += base;
+    const typename Elem<T>::real sc = Elem<T>::bc(scale);
+    auto put = [&](cx<T>* g, int i, int64_t step) {
+        const bool ok0 = tile.ok(i, 0), ok1 = tile.ok(i, 1);
+        cx<T>* h = g + tile.second;
+        return [=](int r, el<T> v) {
+            v = Elem<T>::make(vmul(Elem<T>::re(v), sc), vmul(Elem<T>::im(v), sc));
+            if (ok0) g[r * step] = Elem<T>::template line<0>(v);
+            if (Elem<T>::lines > 1 && ok1) h[r * step] = Elem<T>::template line<1>(v);
+        };
+    };
+    if constexpr (DIR < 0) {
+        stage_first<T, DIR>(buf, p, lay, tw,
+                            [&](int i, int j, int m) { return tile.get(in + i + j * es, i, m * es); });
+        __syncthreads();
+        stages_mid<T, DIR>(buf, p, lay, tw);
+        stage_last<T, DIR>(buf, p, lay, tw, tab + p.rev,
+                           [&](int i, int k0) { return put(out + i + k0 * es, i, p.kstep * es); });
+    } else {
+        stage_in<T, DIR>(buf, p, lay, tw, tab + p.rev,
+                         [&](int i, int k0) { return tile.get(in + i + k0 * es, i, p.kstep * es); });
+        __syncthreads();
+        stages_back<T, DIR>(buf, p, lay, tw);
+        stage_out<T, DIR>(buf, p, lay, tw,
+                          [&](int i, int j, int m) { return put(out + i + j * es, i, m * es); });
+    }
+}
+
+// ---------------------------------------------------------------------------------
+// rows: real <-> half spectrum along x.  Even nx packs x[2m], x[2m+1] into one
+// complex and runs an nx/2-point FFT with the split/merge twiddles W_nx^k; odd nx
+// runs the full nx-point complex FFT.
+// ---------------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ el<T> r2c_post(el<T> zk, el<T> zm, el<T> w) {
+    // X[k] = 1/2 (Z[k] + conj Z[M-k]) - i/2 W^k (Z[k] - conj Z[M-k])
+    using E = Elem<T>;
+    const el<T> s = E::make(vadd(E::re(zk), E::re(zm)), vsub(E::im(zk), E::im(zm)));
+    const el<T> d = E::make(vsub(E::re(zk), E::re(zm)), vadd(E::im(zk), E::im(zm)));
+    return CE<T>::scale(CE<T>::template addi<-1>(s, CE<T>::template cmulw<-1>(d, w)), 0.5);
+}
+template <typename T>
+__device__ __forceinline__ el<T> c2r_pre(el<T> xk, el<T> xm, el<T> w) {
+    // Z[k] = (X[k] + conj X[M-k]) + i W^-k (X[k] - conj X[M-k]); IFFT_M(Z) = nx * (x[2m] + i x[2m+1])
+    using E = Elem<T>;
+    const el<T> e = E::make(vadd(E::re(xk), E::re(xm)), vsub(E::im(xk), E::im(xm)));
+    const el<T> d = E::make(vsub(E::re(xk), E::re(xm)), vadd(E::im(xk), E::im(xm)));
+    return CE<T>::template addi<1>(e, CE<T>::template cmulw<1>(d, w));
+}
+// The stepper's cubic term (psi3_split.hpp:8-13 with the stabilisation constant C)
+template <typename R>
+__device__ __forceinline__ R cubic(R v, R mul, R nC, R nmu) {  // nC = -C, nmu = -mu
+    const R t = vmul(v, mul);
+    return vfma(vfma(t, t, nC), t, nmu);
+}
+
+// kR2C: real rows (in) to half-spectrum rows (out); kC2R: half-spectrum rows to real rows;
+// kNonlin: the stepper's x pass, C2R, the cubic nonlinearity, R2C, in place on rows of the
+// mixed (kx, y, z) field (in == out).  A CTA owns rpc lines of
+// the engine: whole rows (FP64) or pairs of rows (FP32).  The transforms leave
+// frequencies (or cells) digit-reversed; the R2C merge and the C2R output read them back in
+// natural order through the position table, so that global accesses stay contiguous.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
+    k_rows(const void* in, void* out, int nrows, int nx, const __grid_constant__ GPlan p,
+           const el<T>* __restrict__ tw, const int* __restrict__ tab, const el<T>* __restrict__ post, int rpc,
+           double mul, double C, double mu, int64_t ms, FastDiv by_nxh) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
+    constexpr int W = Elem<T>::lines;
+    const int row0 = blockIdx.x * rpc * W;
+    const int nr = min(rpc * W, nrows - row0), nl = (nr + W - 1) / W;
+    const RowLines lay{nl, p.np};
+    const int L = p.n, nxh = nx / 2 + 1;
+    const bool even = (nx & 1) == 0;
+    const int* pos = tab + p.pos;
+    // the second row of an odd last pair repeats the first (and is not stored)
+    auto second = [&](int i, int64_t len) { return W > 1 && 2 * i + 1 < nr ? len : 0; };
+    if (MODE == kR2C) {
+        const T* rows = static_cast<const T*>(in) + (int64_t)row0 * nx;
+        stage_first<T, -1>(buf, p, lay, tw, [&](int i, int j, int m) {
+            const T* a = rows + (int64_t)(W * i) * nx;
+            const T* b = a + second(i, nx);
+            return [=](int r) {
+                const int k = j + r * m;
+                if (even)
+                    return Elem<T>::pack(reinterpret_cast<const cx<T>*>(a)[k], reinterpret_cast<const cx<T>*>(b)[k]);
+                return Elem<T>::pack(mkc<T>(a[k], T(0)), mkc<T>(b[k], T(0)));
+            };
+        });
+    } else {
+        const cx<T>* rows = static_cast<const cx<T>*>(in) + blockIdx.z * ms + (int64_t)row0 * nxh;  // grid z: batch
+        stage_first<T, 1>(buf, p, lay, tw, [&](int i, int j, int m) {
+            const cx<T>* a = rows + (int64_t)(W * i) * nxh;
+            const cx<T>* b = a + second(i, nxh);
+            return [=](int r) {
+                const int k = j + r * m;
+                if (even)
+                    return c2r_pre<T>(Elem<T>::pack(a[k], b[k]), Elem<T>::pack(a[L - k], b[L - k]), post[k]);
+                return k < nxh ? Elem<T>::pack(a[k], b[k]) : Elem<T>::pack(cconj(a[nx - k]), cconj(b[nx - k]));
+            };
+        });
+    }
+    __syncthreads();
+    if (MODE == kR2C) {
+        stages_mid<T, -1>(buf, p, lay, tw);
+        stage_inplace<T, -1, false, false>(buf, p, p.nst - 1, lay, tw);
+        __syncthreads();
+    } else {
+        stages_mid<T, 1>(buf, p, lay, tw);
+    }
+    if (MODE == kC2R) {
+        stage_inplace<T, 1, false, false>(buf, p, p.nst - 1, lay, tw);
+        __syncthreads();
+        T* rows = static_cast<T*>(out) + (int64_t)row0 * nx;
+        for (int e = threadIdx.x; e < nl * L; e += blockDim.x) {
+            const int i = fdiv(e, p.by_n), m = e - i * L;
+            const el<T> v = buf[i * p.np + pos[m]];
+            T* a = rows + (int64_t)(W * i) * nx;
+            auto put = [&](T* row, cx<T> z) {
+                if (even) reinterpret_cast<cx<T>*>(row)[m] = z;
+                else row[m] = z.x;
+            };
+            put(a, Elem<T>::template line<0>(v));
+            if (W > 1 && 2 * i + 1 < nr) put(a + nx, Elem<T>::template line<1>(v));
+        }
+        return;
+    }
+    if (MODE == kNonlin) {
+        // the last inverse stage, the cubic term and the first forward stage on one set of
+        // registers: cells rev[b] + r kstep of the row
+        const auto bmul = Elem<T>::bc(mul), nC = Elem<T>::bc(-C), nmu = Elem<T>::bc(-mu);
+        const GStage& s = p.st[p.nst - 1];
+        const int total = lay.count(p.kstep);
+        by_radix(s.R, [&](auto RC) {
+            constexpr int R = decltype(RC)::value;
+            if constexpr (R > 0) {
+                for (int e = threadIdx.x; e < total; e += blockDim.x) {
+                    int i, b;
+                    lay.split(e, p.kstep, s.by_nb, i, b);
+                    el<T>* a = buf + lay.at(i, b * s.Ms);
+                    el<T> v[R];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) v[r] = a[r];
+                    EDft<T, 1, R>::run(v);
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        v[r] = Elem<T>::make(cubic(Elem<T>::re(v[r]), bmul, nC, nmu),
+                                             even ? cubic(Elem<T>::im(v[r]), bmul, nC, nmu) : Elem<T>::bc(0.0));
+                    EDft<T, -1, R>::run(v);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r] = v[r];
+                }
+            }
+        });
+        __syncthreads();
+        stages_back<T, -1>(buf, p, lay, tw);
+        stage_inplace<T, -1, true, true>(buf, p, 0, lay, tw);
+        __syncthreads();
+    }
+    // the merge, in the order of the frequencies: natural after the transform back (kNonlin),
+    // through the position table otherwise
+    cx<T>* rows = static_cast<cx<T>*>(out) + blockIdx.z * ms + (int64_t)row0 * nxh;
+    auto at = [&](int k) { return MODE == kNonlin ? gpad(p, k) : pos[k]; };
+    for (int e = threadIdx.x; e < nl * nxh; e += blockDim.x) {
+        const int i = fdiv(e, by_nxh), k = e - i * nxh;
+        const el<T>* y = buf + i * p.np;
+        el<T> v;
+        if (even) v = r2c_post<T>(y[at(k == L ? 0 : k)], y[at(k == 0 ? 0 : L - k)], post[k]);
+        else v = y[at(k)];
+        cx<T>* a = rows + (int64_t)(W * i) * nxh + k;
+        a[0] = Elem<T>::template line<0>(v);
+        if (W > 1 && 2 * i + 1 < nr) a[nxh] = Elem<T>::template line<1>(v);
+    }
+}
+
+}  // namespace
+
+template <typename T> cudaError_t gen_attrs() {
+    const int m = (int)kMaxDynSmem;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_cols<T, -1>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_cols<T, 1>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_rows<T, kR2C>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_rows<T, kC2R>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_rows<T, kNonlin>, attr, m);
+    return e;
+}
+
+template <typename T>
+cudaError_t gen_cols(const pfc_ctx* c, int axis, int dir, const void* in, void* out, double scale) {
+    const AxisPlan& ap = axis == 1 ? c->py : c->pz;
+    const int n = ap.plan.n;
+    if (n == 1 && in == out && scale == 1.0) return cudaSuccess;
+    int64_t es, os;
+    int no;
+    if (axis == 1) { es = c->nxh; os = (int64_t)c->ny * c->nxh; no = c->nz; }
+    else { es = (int64_t)c->ny * c->nxh; os = c->nxh; no = c->ny; }
+    const int tile = Elem<T>::lines << ap.lg;
+    dim3 grid((c->nxh + tile - 1) / tile, no, c->batch);
+    auto k = dir < 0 ? k_cols<T, -1> : k_cols<T, 1>;
+    k<<<grid, ap.threads, ap.smem, c->stream>>>((const cx<T>*)in, (cx<T>*)out, c->nxh, es, os, ap.plan,
+                                                (const el<T>*)c->gtw, c->fft_tab, ap.lg, scale, c->mstride);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t gen_rows(const pfc_ctx* c, int mode, const void* in, void* out, double mul, double C, double mu) {
+    const AxisPlan& ap = c->px;
+    const int nrows = c->ny * c->nz;
+    const el<T>* tw = (const el<T>*)c->gtw;
+    const int rows = ap.lines * Elem<T>::lines;
+    // (the plain transforms run on one field; the x pass on all fields of a batch)
+    dim3 grid((nrows + rows - 1) / rows, 1, mode == kNonlin ? c->batch : 1);
+    auto k = mode == kR2C ? k_rows<T, kR2C> : mode == kC2R ? k_rows<T, kC2R> : k_rows<T, kNonlin>;
+    k<<<grid, ap.threads, ap.smem, c->stream>>>(in, out, nrows, c->nx, ap.plan, tw, c->fft_tab, tw + c->post_off,
+                                                ap.lines, mul, C, mu, c->mstride, make_fastdiv(c->nxh));
+    return cudaGetLastError();
+}
+}  // namespace pfc

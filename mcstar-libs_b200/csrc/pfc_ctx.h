@@ -5,6 +5,7 @@
 #include <string>
 #include <utility>
 #include <vector>
+#include "genfft.cuh"
 #include "pfc_internal.cuh"
 #include "../../include/pfc_b200.h"
 
@@ -16,9 +17,11 @@ constexpr int kRedBlocks = 1184;        // 8 x 148 SMs: fixed grid of the FP64 r
 constexpr int kPeakBlock = 256;         // cells per block of the peak finder
 
 struct AxisPlan {
-    LinePlan plan;
-    int tile;          // lines per CTA (columns) or rows per CTA (x axis)
-    size_t smem;       // dynamic shared memory of the kernel using this plan
+    GPlan plan;
+    int lg;            // 2^lg elements per position and CTA (y, z): columns, in FP32 pairs of columns
+    int lines;         // engine lines per CTA (x): rows, in FP32 pairs of rows
+    int threads;
+    size_t smem;       // dynamic shared memory of the CTA's lines
 };
 
 }  // namespace pfc
@@ -35,9 +38,11 @@ struct pfc_ctx {
 
     pfc::AxisPlan px;             // x: complex length nx/2 (even nx) or nx (odd nx)
     pfc::AxisPlan py, pz;         // y, z: complex length ny, nz
-    pfc::AxisPlan pzprop;         // the stepper's z pass (two fields per tile)
-    pfc::AxisPlan pxnl;           // the stepper's fused x pass
-    int post_off;                 // twiddle offset of W_nx^k, k = 0..nx/2 (even nx)
+    pfc::AxisPlan pzprop, pz2;    // the stepper's z pass carrying psi^; carrying A (two lines per column)
+    pfc::AxisPlan py2;            // the stepper's update pass along the y columns of a 2D field
+    int* fft_tab;                 // device int tables of the plans (GPlan::rev, pos)
+    void* gtw;                    // device twiddles of the general passes (16-byte elements, genfft.cuh)
+    int post_off;                 // its offset of W_nx^k, k = 0..nx/2 (even nx)
     void* tw;                     // device twiddles, cx<F>
     void* work;                   // state_bytes: C2R scratch and the stepper's second field
     void* work2;                  // state_bytes: free-energy real field
@@ -121,7 +126,7 @@ cudaError_t set_fft_attributes(const pfc_ctx* c);
 cudaError_t launch_cols(const pfc_ctx* c, int axis, int dir, const void* in, void* out, double scale);
 cudaError_t launch_rows_r2c(const pfc_ctx* c, const void* in_real, void* out_cmpl);
 cudaError_t launch_rows_c2r(const pfc_ctx* c, const void* in_cmpl, void* out_real);
-cudaError_t launch_rows_nonlin(const pfc_ctx* c, void* buf, const void* pot, double mul, double C, double mu);
+cudaError_t launch_rows_nonlin(const pfc_ctx* c, void* buf, double mul, double C, double mu);
 struct ZPropArgs {
     double dt, eps, C, namp_eff, lx, ly, lz;
     uint64_t seed, counter;
@@ -139,12 +144,10 @@ struct ZPropArgs {
     // context's ky = 0 is the field's ky0, of ny_global rows (0, 0: the context's own field)
     int ky0, ny_global;
 };
+// the general z pass carrying A = IFFT_z(psi^)/nz: A' (or psi^' on the last step) over A
 cudaError_t launch_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs& a);
-// the general z pass over the kx columns [col0, col0 + ncols); carry: A holds psi^ itself
-// (updated in place) and A' = IFFT_z(psi^')/nz goes to anext (not on the final step)
-cudaError_t launch_zprop_cols(const pfc_ctx* c, void* A, const void* B, const ZPropArgs& a, int col0, int ncols,
-                              void* anext = nullptr, bool carry = false);
-// the psi^-carrying general z pass over the whole field (nz > 1)
+// the general pass carrying psi^ itself (updated in place), along z or, in a 2D field, along
+// y: A' = IFFT(psi^')/n goes to anext (which may be B; not on the final step)
 cudaError_t launch_zprop_carry(const pfc_ctx* c, void* kpsi, const void* B, void* anext, const ZPropArgs& a);
 
 // ---- register-resident y and x passes (kern_passes.cu) ----

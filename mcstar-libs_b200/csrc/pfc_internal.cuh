@@ -1,6 +1,5 @@
 // Internal building blocks of libpfc_b200: complex helpers, small-radix DFTs, the
-// shared-memory Stockham line FFT used by the general-size kernels, the wavenumber
-// of the reference, Philox4x32-10 and the noise draw.
+// wavenumber of the reference, Philox4x32-10 and the noise draw.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -89,16 +88,6 @@ template <typename T, int DIR> struct Dft<T, DIR, 5> {
     }
 };
 
-// ---------------------------------------------------------------------------------
-// Stockham autosort FFT over lines held in shared memory (general 2^a 3^b 5^c).
-// Stage s has radix R_s and span Ns = R_0 ... R_{s-1}: butterfly j reads
-// x[j + r n/R], applies exp(DIR 2 pi i r (j mod Ns) / (Ns R)), runs the R-point DFT
-// and writes to (j - j mod Ns) R + j mod Ns + r Ns.  Twiddles are precomputed on
-// the host in FP64 (forward sign; the inverse uses their conjugates).
-// ---------------------------------------------------------------------------------
-constexpr int kMaxStages = 16;
-constexpr int kMaxOddRadix = 31;  // largest prime radix of the general stage
-
 // Division of a non-negative 31-bit n by a fixed d >= 1 as a multiply-high, an add and a
 // shift: with l = ceil(log2 d) and mul = floor(2^32 (2^l - d) / d) + 1 (below 2^32),
 // n / d = (umulhi(n, mul) + n) >> l for every n < 2^31 (the round-up method of Granlund and
@@ -115,113 +104,6 @@ __host__ __device__ inline FastDiv make_fastdiv(int d) {
 }
 __device__ __forceinline__ int fdiv(int n, FastDiv f) {
     return (int)((__umulhi((uint32_t)n, f.mul) + (uint32_t)n) >> f.shift);
-}
-
-// Lines of the Stockham engine in shared memory: element k of a line sits at lpad(k) (one
-// pad element after every 32), so that the strided writes of the early stages (R apart) and
-// the reads of later ones spread over the banks; lines are line_stride(n) elements apart, an
-// odd number, so that the lanes of a warp moving one element of each of consecutive lines
-// hit distinct banks too.
-__host__ __device__ __forceinline__ constexpr int lpad(int k) { return k + (k >> 5); }
-__host__ __device__ constexpr int line_stride(int n) { return (n + (n >> 5) + 1) | 1; }
-
-struct LinePlan {
-    int n;
-    int nst;
-    int radix[kMaxStages];
-    int ns[kMaxStages];
-    int twoff[kMaxStages];
-    int rtoff[kMaxStages];     // W_R^q, q < R, for radices without a hand-written DFT
-    FastDiv by_n;              // division by n
-    FastDiv by_m[kMaxStages];  // by n / R_s
-    FastDiv by_ns[kMaxStages]; // by Ns
-};
-
-// Stage of a prime radix R (7 <= R <= kMaxOddRadix): direct R-point DFT with the
-// roots of unity W_R^q from the plan's table.
-template <typename T, int DIR>
-__device__ __forceinline__ void stockham_bfly_gen(const cx<T>* __restrict__ sl, cx<T>* __restrict__ dl, int j,
-                                                  int m, int Ns, int R, const cx<T>* __restrict__ tws,
-                                                  const cx<T>* __restrict__ wr, FastDiv by_ns) {
-    cx<T> v[kMaxOddRadix];
-    const int jj = j - fdiv(j, by_ns) * Ns;
-    for (int r = 0; r < R; ++r) {
-        cx<T> a = sl[lpad(j + r * m)];
-        if (Ns > 1 && r > 0) {
-            cx<T> w = tws[jj * (R - 1) + r - 1];
-            if (DIR > 0) w.y = -w.y;
-            a = cmul(a, w);
-        }
-        v[r] = a;
-    }
-    const int od = (j - jj) * R + jj;
-    for (int k = 0; k < R; ++k) {
-        cx<T> acc = v[0];
-        int q = 0;
-        for (int r = 1; r < R; ++r) {
-            q += k;
-            if (q >= R) q -= R;
-            cx<T> w = wr[q];
-            if (DIR > 0) w.y = -w.y;
-            const cx<T> p = cmul(v[r], w);
-            acc.x += p.x;
-            acc.y += p.y;
-        }
-        dl[lpad(od + k * Ns)] = acc;
-    }
-}
-
-template <typename T, int DIR, int R>
-__device__ __forceinline__ void stockham_bfly(const cx<T>* __restrict__ sl, cx<T>* __restrict__ dl,
-                                              int j, int m, int Ns, const cx<T>* __restrict__ tws,
-                                              FastDiv by_ns) {
-    cx<T> v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = sl[lpad(j + r * m)];
-    const int jj = j - fdiv(j, by_ns) * Ns;
-    if (Ns > 1) {
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            cx<T> w = tws[jj * (R - 1) + r - 1];
-            if (DIR > 0) w.y = -w.y;
-            v[r] = cmul(v[r], w);
-        }
-    }
-    Dft<T, DIR, R>::run(v);
-    const int od = (j - jj) * R + jj;
-#pragma unroll
-    for (int r = 0; r < R; ++r) dl[lpad(od + r * Ns)] = v[r];
-}
-
-// FFT of nlines lines, line l at a[l*ld .. l*ld+n).  Ping-pongs between a and b and
-// returns the buffer holding the result.  All threads of the block must call it.
-template <typename T, int DIR>
-__device__ cx<T>* stockham_lines(cx<T>* a, cx<T>* b, int nlines, int ld, const LinePlan& p,
-                                 const cx<T>* __restrict__ tw) {
-    cx<T>* src = a;
-    cx<T>* dst = b;
-    for (int s = 0; s < p.nst; ++s) {
-        const int R = p.radix[s], Ns = p.ns[s], m = p.n / R;
-        const FastDiv by_m = p.by_m[s], by_ns = p.by_ns[s];
-        const cx<T>* tws = tw + p.twoff[s];
-        const int total = nlines * m;
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-            const int line = fdiv(e, by_m), j = e - line * m;
-            const cx<T>* sl = src + (size_t)line * ld;
-            cx<T>* dl = dst + (size_t)line * ld;
-            switch (R) {
-                case 8: stockham_bfly<T, DIR, 8>(sl, dl, j, m, Ns, tws, by_ns); break;
-                case 4: stockham_bfly<T, DIR, 4>(sl, dl, j, m, Ns, tws, by_ns); break;
-                case 2: stockham_bfly<T, DIR, 2>(sl, dl, j, m, Ns, tws, by_ns); break;
-                case 3: stockham_bfly<T, DIR, 3>(sl, dl, j, m, Ns, tws, by_ns); break;
-                case 5: stockham_bfly<T, DIR, 5>(sl, dl, j, m, Ns, tws, by_ns); break;
-                default: stockham_bfly_gen<T, DIR>(sl, dl, j, m, Ns, R, tws, tw + p.rtoff[s], by_ns); break;
-            }
-        }
-        __syncthreads();
-        cx<T>* t = src; src = dst; dst = t;
-    }
-    return src;
 }
 
 // ---------------------------------------------------------------------------------

@@ -189,7 +189,7 @@ extern "C" pfc_status pfc_tune(const pfc_desc* d, const char* cache_path, pfc_op
         pfc_ctx* c = nullptr;
         pfc_status s = pfc_create_with(d, &cur, &c);
         if (s != PFC_OK) return s;
-        general = c->xy_mode != 2 || (c->nz > 1 && !c->fused_z);
+        general = c->xy_mode != 2 || c->nz == 1 || !c->fused_z;
         zcarry_ok = c->nz > 1;  // (both z passes carry either state)
         xks = c->fused_x ? pfc::xkernel_variants(c->nx, c->dtype) : 1;
         tiled_ok = c->fused_z && c->fused_zfft && c->xy_mode == 2 && c->fused_y;

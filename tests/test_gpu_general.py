@@ -1,0 +1,67 @@
+"""The general-length passes (csrc/genfft.cuh): plain transforms and steps at the lengths where
+the engine's stages, padding and tiles can go wrong -- prime radices (with the appended stage of
+radix 1), odd and even last radices, one to five stages, odd row lengths (a last unpaired row in
+FP32), partial last column tiles, one-mode-wide fields -- against numpy in FP64.
+
+Tolerances: a transform of n points does about log2 n roundings per value, each within half
+an ulp (2^-24, 2^-53) of the running value and independent: the relative L2 error stays below
+log2(n) ulps with a factor to spare over its sqrt(log2 n) expectation."""
+import math
+
+import numpy as np
+import pytest
+
+import pfc_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+F32, F64 = np.float32, np.float64
+SHAPES = [(7, 5, 3), (14, 9, 1), (26, 31, 4), (2, 2, 2), (1, 6, 4), (15, 1, 1), (62, 49, 5), (30, 24, 18), (34, 27, 25),
+          (66, 50, 36), (121, 100, 1), (250, 240, 3), (90, 81, 80), (400, 375, 1), (2000, 7, 1), (22, 1280, 1),
+          (1458, 625, 1), (720, 36, 11)]
+
+
+def rel(a, b):
+    return float(np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel()))
+
+
+@pytest.mark.parametrize("dtype", [F32, F64], ids=["f32", "f64"])
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+def test_general_transforms(shape, dtype):
+    from mcstar_b200 import C2R, R2C, CPUArray, CufftPlan, GPUArray
+    nx, ny, nz = shape
+    x = np.random.default_rng(5).uniform(-1, 1, (nz, ny, nx)).astype(dtype)
+    want = np.fft.rfftn(x.astype(F64), axes=(0, 1, 2))
+    tol = max(1.0, math.log2(x.size)) * (2.0 ** -24 if dtype == F32 else 2.0 ** -53)
+    h = CPUArray(shape, dtype)
+    h.numpy()[: x.size] = x.ravel()
+    a, k, b = GPUArray(h), GPUArray(shape, dtype), GPUArray(shape, dtype)
+    CufftPlan(dtype, R2C, shape).execute(a, k)
+    assert rel(k.ptr_cmpl().cpu().numpy(), want) < tol
+    CufftPlan(dtype, C2R, shape).execute(k, b)
+    assert rel(b.ptr_real().cpu().numpy() / x.size, x) < 2 * tol
+
+
+STEPS = [((121, 100, 1), F32), ((15, 1, 1), F64), ((400, 375, 1), F64), ((34, 27, 25), F32), ((66, 50, 36), F64),
+         ((62, 49, 5), F32), ((96, 96, 96), F32)]
+
+
+@pytest.mark.parametrize("shape,dtype", STEPS, ids=str)
+def test_general_steps_and_resume(shape, dtype):
+    """Steps with noise against the oracle, and a run cut in two repeating its bits (the entry
+    transform of a call is the inverse transform of the step before it)."""
+    from mcstar_b200 import Stepper
+    nx, ny, nz = shape
+    psi = -0.2 + 0.1 * np.random.default_rng(6).uniform(-1, 1, (nz, ny, nx))
+    k0 = O.r2c(psi)
+    runs = []
+    for cuts in ((5,), (2, 3)):
+        st = Stepper(shape, math.pi / 4, 0.5, 0.3, dtype=dtype, namp=0.03, seed=11)
+        st.set_kspace(k0.astype(np.complex64 if dtype == F32 else np.complex128))
+        for n in cuts:
+            st.step(n)
+        runs.append(st.kspace())
+    want = O.step(k0, 5, 0.5, 0.3, st.lens, shape, namp=0.03, seed=11, noise_dtype=dtype)
+    assert rel(runs[0], want) < (2e-6 if dtype == F32 else 1e-12)
+    assert np.array_equal(runs[0], runs[1])
+    assert runs[0][0, 0, 0] == k0.astype(runs[0].dtype)[0, 0, 0]
