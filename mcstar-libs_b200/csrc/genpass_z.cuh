@@ -34,11 +34,6 @@ __device__ __forceinline__ void zmember(ZArgsT<T>& a) {
     }
 }
 
-// The wavenumber of index i of n (common.hpp:27-28), ck = 2 pi / L
-template <typename T> __device__ __forceinline__ T kwave_ck(int i, int n, T ck) {
-    return T(i < n / 2 + 1 ? i : i - n) * ck;
-}
-
 // What a kx column contributes to the modes of a CTA: its wavenumber and kx^2 + ky^2.
 template <typename T> struct ZColumn {
     int kx;
@@ -71,8 +66,8 @@ __device__ __forceinline__ cx<T> zmode_of(cx<T> psi, cx<T> nl, const ZColumn<T>&
         const T f = a.dt * dopx;
         cx<T> num = mkc<T>(psi.x + f * nl.x, psi.y + f * nl.y);
         if (a.use_noise) {
-            const cx<T> xi = kspace_noise<T>(kx, kyg, kz, nx, a.nyg, nz, a.seed, a.counter);
-            const T g = a.dt * a.namp_eff * sqrt(-dopx);
+            const cx<T> xi = kspace_noise<T>(kx, kyg, kz, nx, a.nyg, nz, a.seed, a.counter, kKspaceDomain, -dopx);
+            const T g = a.dt * a.namp_eff;
             num.x += g * xi.x;
             num.y += g * xi.y;
         }

@@ -128,16 +128,17 @@ __device__ __forceinline__ void noise_gain_xi(int kz, int kx, int ky, float kxy,
                                               int ny, const ZArgsF& a, uint64_t ctr, float& g, float2& xi) {
     const float k2z = kz_tab[kz_slot(kz)];
     const float dopx = -kxy - k2z * k2z;
+    float v = 1.0f;
     if constexpr (PROP == kPropConserved) {
         const float dopy = dopx * dopx;
-        const float inv = prop_inv(1.0f - a.dt * (deps * dopx + 2.0f * dopy + dopx * dopy));
-        g = a.dt * a.namp_eff * sqrtf(-dopx) * inv;
+        g = a.dt * a.namp_eff * prop_inv(1.0f - a.dt * (deps * dopx + 2.0f * dopy + dopx * dopy));
+        v = -dopx;  // |k| xi with one square root
     } else {
         float ca, cb, cg;
         prop_coef<PROP, float>(dopx, a.dt, deps, ca, cb, cg);
         g = a.namp_eff * cg;
     }
-    xi = kspace_noise<float>(kx, ky, kz, nx, ny, Z::NZ, a.seed, ctr);
+    xi = kspace_noise<float>(kx, ky, kz, nx, ny, Z::NZ, a.seed, ctr, kKspaceDomain, v);
 }
 
 // noise_modes: the thread's modes m < noise_modes (mode m: kz = (t U + m / P) + E (m % P),
@@ -381,17 +382,17 @@ __device__ __forceinline__ void propagate3(float2 (&v)[Z::E], float2* tile, int 
             const int kz = kzb + off;
             const float k2z = tab[off + (r >= E / 2 ? 2 : 0)];
             const float dopx = -kxy - k2z * k2z;
-            float g;
+            float g, v = 1.0f;
             if constexpr (PROP == kPropConserved) {
                 const float dopy = dopx * dopx;
-                const float inv = prop_inv(1.0f - a.dt * (deps * dopx + 2.0f * dopy + dopx * dopy)) * sc;
-                g = a.dt * a.namp_eff * sqrtf(-dopx) * inv;
+                g = a.dt * a.namp_eff * (prop_inv(1.0f - a.dt * (deps * dopx + 2.0f * dopy + dopx * dopy)) * sc);
+                v = -dopx;  // |k| xi with one square root
             } else {
                 float ca, cb, cg;
                 prop_coef<PROP, float>(dopx, a.dt, deps, ca, cb, cg);
                 g = a.namp_eff * cg * sc;
             }
-            const float2 xi = kspace_noise<float>(kx, ky, kz, nx, ny, NZ, a.seed, ctr);
+            const float2 xi = kspace_noise<float>(kx, ky, kz, nx, ny, NZ, a.seed, ctr, kKspaceDomain, v);
             float2 w = trow[row * TX];
             w.x += g * xi.x;
             w.y += g * xi.y;

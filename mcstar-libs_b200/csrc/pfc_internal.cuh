@@ -106,12 +106,43 @@ __device__ __forceinline__ int fdiv(int n, FastDiv f) {
     return (int)((__umulhi((uint32_t)n, f.mul) + (uint32_t)n) >> f.shift);
 }
 
+// Mode (i0, i1, i2) of a linear half-spectrum index: multiplications by reciprocals while the
+// index fits 31 bits (a 64-bit division takes about 60 instructions: 256^3 FP32 k-space noise
+// fill 78 us with two of them per mode, 55 us so).
+struct ModeIndex {
+    int nxh, ny;
+    FastDiv by_nxh, by_ny;
+    bool small;
+    __device__ __forceinline__ void at(int64_t idx, int& i0, int& i1, int& i2) const {
+        if (small) {
+            const int i = (int)idx, r = fdiv(i, by_nxh);
+            i0 = i - r * nxh;
+            i2 = fdiv(r, by_ny);
+            i1 = r - i2 * ny;
+        } else {
+            const int64_t r = idx / nxh;
+            i0 = (int)(idx - r * nxh);
+            i2 = (int)(r / ny);
+            i1 = (int)(r - (int64_t)i2 * ny);
+        }
+    }
+};
+inline ModeIndex mode_index(int nx, int ny, int nz) {
+    const int nxh = nx / 2 + 1;
+    return ModeIndex{nxh, ny, make_fastdiv(nxh), make_fastdiv(ny), (int64_t)nxh * ny * nz < (1ll << 31)};
+}
+
 // ---------------------------------------------------------------------------------
 // The reference's wavenumber, K(i, n, len) = (i < n/2+1 ? i : i-n) * 2pi / len
 // (cuda/kernels/common.hpp:27-28), evaluated in the field's precision.
 // ---------------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ T kwave(int i, int n, T len) {
     return T(i < n / 2 + 1 ? i : i - n) * T(6.283185307179586232) / len;
+}
+
+// The wavenumber of index i of n (common.hpp:27-28), ck = 2 pi / L
+template <typename T> __device__ __forceinline__ T kwave_ck(int i, int n, T ck) {
+    return T(i < n / 2 + 1 ? i : i - n) * ck;
 }
 
 // ---------------------------------------------------------------------------------
@@ -247,57 +278,97 @@ constexpr uint32_t kRealDomain = 0x52454131u;
 constexpr uint32_t kHpfcDomain = 0x48504600u;  // + 1, 2, 3: the three fields of the hpfc noise
 
 
-// Two standard normals from counter (idx, counter) under key (seed, domain),
-// Box-Muller on uniforms strictly inside (0, 1) that are exact in T.
-template <typename T> __device__ __forceinline__ void philox_normal2(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                     uint32_t domain, T& g1, T& g2);
-template <> __device__ __forceinline__ void philox_normal2<float>(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                  uint32_t domain, float& g1, float& g2) {
-    U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
-    U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
+// cos and sin of 2 pi m / 2^53 for an integer 0 <= m < 2^53: the quarter turn nearest the angle
+// is taken off exactly in integers; the rest, f quarter turns with |f| <= 1/2, goes through
+// the Taylor polynomials of cos and sin of (pi/2) f (truncation below 2^-55), the leading
+// coefficient of the sine in two parts.  (sincospi reduces arguments of any size; in FP32
+// the difference measured nothing, so sincospif stays.)
+__device__ __forceinline__ void cos_sin_2pi(uint64_t m, double& co, double& si) {
+    const uint64_t q = (m + (1ull << 50)) >> 51;
+    const double f = (double)(int64_t)(m - (q << 51)) * 4.44089209850062616e-16;  // 2^-51
+    const double t = f * f;
+    double c = 5.2944002007346235e-13;
+    c = fma(t, c, -6.5659631149794728e-11);
+    c = fma(t, c, 6.3866030837918521e-09);
+    c = fma(t, c, -4.7108747788181717e-07);
+    c = fma(t, c, 2.5202042373060607e-05);
+    c = fma(t, c, -9.1926027483942659e-04);
+    c = fma(t, c, 2.0863480763352961e-02);
+    c = fma(t, c, -2.5366950790104803e-01);
+    c = fma(t, c, 1.2337005501361697e+00);
+    c = fma(-t, c, 1.0);
+    double s = -4.3770654673137423e-14;
+    s = fma(t, s, 6.0669357311061956e-12);
+    s = fma(t, s, -6.6880351098114670e-10);
+    s = fma(t, s, 5.6921729219679267e-08);
+    s = fma(t, s, -3.5988432352120852e-06);
+    s = fma(t, s, 1.6044118478735983e-04);
+    s = fma(t, s, -4.6817541353186883e-03);
+    s = fma(t, s, 7.9692626246167048e-02);
+    s = fma(t, s, -6.4596409750624628e-01);
+    s = fma(t, s, 6.1232339957367660e-17);  // pi/2 - 1.5707963267948966
+    s = fma(f, 1.5707963267948966, f * s);
+    const double x = (q & 1) ? s : c, y = (q & 1) ? c : s;
+    co = ((q + 1) & 2) ? -x : x;
+    si = (q & 2) ? -y : y;
+}
+
+// sqrt(-v log u1) (cos, sin)(2 pi u2) from counter (idx, counter) under key (seed, domain),
+// u1 and u2 uniform strictly inside (0, 1) and exact in T (Box-Muller; v = 2 gives two
+// standard normals).
+template <typename T> __device__ __forceinline__ cx<T> philox_polar(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                    uint32_t domain, T v);
+template <> __device__ __forceinline__ float2 philox_polar<float>(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                  uint32_t domain, float v) {
+    const U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
+    const U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
     const float u1 = (float)((r.x >> 9) * 2u + 1u) * 5.9604644775390625e-08f;  // 2^-24
+    const float rad = sqrtf(-v * logf(u1));
     const float u2 = (float)((r.y >> 9) * 2u + 1u) * 5.9604644775390625e-08f;
-    const float rad = sqrtf(-2.0f * logf(u1));
     float s, co;
     sincospif(2.0f * u2, &s, &co);
-    g1 = rad * co; g2 = rad * s;
+    return make_float2(rad * co, rad * s);
 }
-template <> __device__ __forceinline__ void philox_normal2<double>(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                   uint32_t domain, double& g1, double& g2) {
-    U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
-    U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
+template <> __device__ __forceinline__ double2 philox_polar<double>(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                    uint32_t domain, double v) {
+    const U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
+    const U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
     const uint64_t a = ((((uint64_t)r.x << 32) | r.y) >> 12) * 2u + 1u;
     const uint64_t b = ((((uint64_t)r.z << 32) | r.w) >> 12) * 2u + 1u;
     const double u1 = (double)a * 1.1102230246251565404e-16;  // 2^-53
-    const double u2 = (double)b * 1.1102230246251565404e-16;
-    const double rad = sqrt(-2.0 * log(u1));
+    const double rad = sqrt(-v * log(u1));
     double s, co;
-    sincospi(2.0 * u2, &s, &co);
-    g1 = rad * co; g2 = rad * s;
+    cos_sin_2pi(b, co, s);
+    return make_double2(rad * co, rad * s);
+}
+template <typename T> __device__ __forceinline__ void philox_normal2(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                     uint32_t domain, T& g1, T& g2) {
+    const cx<T> g = philox_polar<T>(idx, seed, counter, domain, T(2));
+    g1 = g.x;
+    g2 = g.y;
 }
 
-// k-space noise of half-spectrum mode (i0, i1, i2): modes on the i0 = 0 and
-// i0 = nx/2 planes are keyed by the canonical (lower linear index) member of their
-// +-k pair and conjugated on the other member; self-conjugate modes are real.
+// sqrt(v) times the k-space noise of half-spectrum mode (i0, i1, i2): complex normal with unit
+// variance; modes on the i0 = 0 and i0 = nx/2 planes are keyed by the canonical (lower linear
+// index) member of their +-k pair and conjugated on the other member; self-conjugate modes
+// are real.  (v = k^2 gives the conserved noise |k| xi with one square root.)
 template <typename T>
-__device__ __forceinline__ cx<T> kspace_noise(int i0, int i1, int i2, int nx, int ny, int nz,
-                                              uint64_t seed, uint64_t counter, uint32_t domain = kKspaceDomain) {
-    const int nxh = nx / 2 + 1;
-    const int64_t lin = ((int64_t)i2 * ny + i1) * nxh + i0;
-    int64_t canon = lin;
-    bool conj = false, selfc = false;
-    if (i0 == 0 || ((nx & 1) == 0 && i0 == nx / 2)) {
+__device__ __forceinline__ cx<T> kspace_noise(int i0, int i1, int i2, int nx, int ny, int nz, uint64_t seed,
+                                              uint64_t counter, uint32_t domain = kKspaceDomain, T v = T(1)) {
+    const int nxh = nx / 2 + 1, plane = ny * nxh;  // (a plane's modes fit an int: lengths are at most some 10^4)
+    int64_t key = (int64_t)i2 * plane + (i1 * nxh + i0);
+    T fy = T(1);  // -1 on the conjugate member, 0 on a self-conjugate mode
+    if (i0 == 0 || 2 * i0 == nx) {
         const int j1 = i1 == 0 ? 0 : ny - i1;
         const int j2 = i2 == 0 ? 0 : nz - i2;
-        const int64_t part = ((int64_t)j2 * ny + j1) * nxh + i0;
-        if (part < lin) { canon = part; conj = true; }
-        selfc = (part == lin);
+        const int64_t part = (int64_t)j2 * plane + (j1 * nxh + i0);
+        if (part <= key) fy = part < key ? T(-1) : T(0);
+        if (part == key) v = v * T(2);
+        key = min(key, part);
     }
-    T g1, g2;
-    philox_normal2<T>((uint64_t)canon, seed, counter, domain, g1, g2);
-    const T s = T(0.70710678118654752440);
-    if (selfc) return mkc<T>(g1, T(0));
-    return mkc<T>(g1 * s, conj ? -g2 * s : g2 * s);
+    cx<T> g = philox_polar<T>((uint64_t)key, seed, counter, domain, v);
+    g.y *= fy;
+    return g;
 }
 
 // The anisotropic 2D noise of eom.hpp:16-58 at wavenumbers (k0, k1), |k| = kabs: the three
