@@ -1301,21 +1301,19 @@ pfc_status pfc_adjoint_step(pfc_ctx* ctx, const void* kpsi_n, const void* kpsi_n
     void* w2 = ctx->work2;
     pfc_status s = pfc_fft_r2c(ctx, lam, w1);
     if (s != PFC_OK) return s;
+    PFC_CUDA(launch_adj_spectral(ctx, w1, w2, deps ? kpsi_np1 : nullptr, p), "pfc_adjoint_step K, M, eps");
     if (deps) {
-        PFC_CUDA(launch_adj_eps(ctx, w1, kpsi_np1, p), "pfc_adjoint_step eps");
         double v = 0.0;
         PFC_CUDA(cudaMemcpyAsync(&v, ctx->red + kRedBlocks + 3, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
                  "pfc_adjoint_step copy");
         PFC_CUDA(cudaStreamSynchronize(ctx->stream), "pfc_adjoint_step sync");
         *deps += v;
     }
-    PFC_CUDA(launch_adj_mul(ctx, w1, w2, p, 1), "pfc_adjoint_step K");
     if ((s = pfc_fft_c2r(ctx, w2, w3)) != PFC_OK) return s;
-    PFC_CUDA(launch_adj_mul(ctx, w1, w1, p, 0), "pfc_adjoint_step M");
     if ((s = pfc_fft_c2r(ctx, w1, lam)) != PFC_OK) return s;
     if ((s = pfc_fft_c2r(ctx, kpsi_n, w2)) != PFC_OK) return s;
     PFC_CUDA(launch_adj_combine(ctx, lam, w2, w3, p->C), "pfc_adjoint_step combine");
-    ctx->launches += 4;
+    ctx->launches += deps ? 3 : 2;
     return PFC_OK;
 }
 

@@ -21,20 +21,14 @@ namespace {
 
 struct AdjGeom {
     int nx, ny, nz;
-    double lx, ly, lz, dt, eps, C;
+    double ckx, cky, ckz, dt, eps, C;  // ck = 2 pi / L per axis
+    ModeIndex mi;
 };
-
-__device__ __forceinline__ void mode_of(int64_t idx, int nx, int ny, int& i0, int& i1, int& i2) {
-    const int nxh = nx / 2 + 1;
-    i0 = (int)(idx % nxh);
-    const int64_t r = idx / nxh;
-    i1 = (int)(r % ny);
-    i2 = (int)(r / ny);
-}
 
 // 1/D and dt k^2 / D at mode (i0, i1, i2)
 __device__ __forceinline__ void prop_factors(const AdjGeom& g, int i0, int i1, int i2, double& inv_d, double& kfac) {
-    const double k0 = kwave<double>(i0, g.nx, g.lx), k1 = kwave<double>(i1, g.ny, g.ly), k2 = kwave<double>(i2, g.nz, g.lz);
+    const double k0 = kwave_ck<double>(i0, g.nx, g.ckx), k1 = kwave_ck<double>(i1, g.ny, g.cky),
+                 k2 = kwave_ck<double>(i2, g.nz, g.ckz);
     const double k2s = k0 * k0 + k1 * k1 + k2 * k2;
     const double om = 1.0 - k2s;
     inv_d = 1.0 / (1.0 + g.dt * k2s * (g.C - g.eps + om * om));
@@ -56,38 +50,29 @@ __device__ __forceinline__ void block_sum(double s, double* out) {
     if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
-// out = (1/D) in (mode 0) or (dt k^2 / D) in (mode 1); in may equal out
+// From lam^ (in w): M lam^ = lam^ / D over it and K lam^ = (dt k^2 / D) lam^ into kl, one FP64
+// division per mode for both; with p (psi^ of the step's end) also the block partials of
+// sum_k w_k Re(conj(lam^_k) (dt k^2 / D_k) p_k).
 template <typename T>
-__global__ void k_adj_mul(const cx<T>* in, cx<T>* out, AdjGeom g, int mode) {
-    const int64_t total = (int64_t)(g.nx / 2 + 1) * g.ny * g.nz;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i0, i1, i2;
-        mode_of(idx, g.nx, g.ny, i0, i1, i2);
-        double inv_d, kfac;
-        prop_factors(g, i0, i1, i2, inv_d, kfac);
-        const double f = mode ? kfac : inv_d;
-        const cx<T> v = in[idx];
-        out[idx] = mkc<T>((T)(f * (double)v.x), (T)(f * (double)v.y));
-    }
-}
-
-// block partials of sum_k w_k Re(conj(lh_k) (dt k^2 / D_k) p_k)
-template <typename T>
-__global__ void __launch_bounds__(256) k_adj_eps(const cx<T>* __restrict__ lh, const cx<T>* __restrict__ p, AdjGeom g,
-                                                 double* __restrict__ partial) {
+__global__ void __launch_bounds__(256) k_adj_spectral(cx<T>* w, cx<T>* __restrict__ kl, const cx<T>* __restrict__ p,
+                                                      AdjGeom g, double* __restrict__ partial) {
     const int64_t total = (int64_t)(g.nx / 2 + 1) * g.ny * g.nz;
     double s = 0.0;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
         int i0, i1, i2;
-        mode_of(idx, g.nx, g.ny, i0, i1, i2);
+        g.mi.at(idx, i0, i1, i2);
         double inv_d, kfac;
         prop_factors(g, i0, i1, i2, inv_d, kfac);
-        const cx<T> a = lh[idx], b = p[idx];
-        s += half_weight(i0, g.nx) * kfac * ((double)a.x * b.x + (double)a.y * b.y);
+        const cx<T> a = w[idx];
+        if (p) {
+            const cx<T> b = p[idx];
+            s += half_weight(i0, g.nx) * kfac * ((double)a.x * b.x + (double)a.y * b.y);
+        }
+        kl[idx] = mkc<T>((T)(kfac * (double)a.x), (T)(kfac * (double)a.y));
+        w[idx] = mkc<T>((T)(inv_d * (double)a.x), (T)(inv_d * (double)a.y));
     }
-    block_sum(s, partial);
+    if (p) block_sum(s, partial);
 }
 
 // lam <- (A - (3 (psi_u / N)^2 - C) B) / N, A (in lam), psi_u and B unnormalised C2R outputs
@@ -104,14 +89,14 @@ __global__ void k_adj_combine(T* __restrict__ lam, const T* __restrict__ psi_u, 
 template <typename T>
 __global__ void __launch_bounds__(256) k_sf_loss(const cx<T>* __restrict__ kpsi, const T* __restrict__ s_target,
                                                  cx<T>* __restrict__ out, int nx, int ny, int nz,
-                                                 double* __restrict__ partial) {
+                                                 ModeIndex mi, double* __restrict__ partial) {
     const int64_t total = (int64_t)(nx / 2 + 1) * ny * nz;
     const double inv_n = 1.0 / ((double)nx * ny * nz);
     double s = 0.0;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
         int i0, i1, i2;
-        mode_of(idx, nx, ny, i0, i1, i2);
+        mi.at(idx, i0, i1, i2);
         const cx<T> v = kpsi[idx];
         const double r = ((double)v.x * v.x + (double)v.y * v.y) * inv_n - (double)s_target[idx];
         s += half_weight(i0, nx) * r * r;
@@ -128,29 +113,23 @@ inline int grid_for(size_t n, int block) {
 }
 
 AdjGeom geom(const pfc_ctx* c, const pfc_step_params* p) {
-    return AdjGeom{c->nx, c->ny, c->nz, p->lx, p->ly, p->lz, p->dt, p->eps, p->C};
+    const double tp = 6.283185307179586232;
+    return AdjGeom{c->nx, c->ny, c->nz, tp / p->lx, tp / p->ly, tp / p->lz, p->dt, p->eps, p->C,
+                   mode_index(c->nx, c->ny, c->nz)};
 }
 
 }  // namespace
 
-cudaError_t launch_adj_mul(const pfc_ctx* c, const void* in, void* out, const pfc_step_params* p, int mode) {
-    const int g = grid_for(c->n_cmpl, 256);
+cudaError_t launch_adj_spectral(const pfc_ctx* c, void* w, void* kl, const void* kpsi_np1,
+                                const pfc_step_params* p) {
     if (c->dtype == PFC_F64)
-        k_adj_mul<double><<<g, 256, 0, c->stream>>>((const cx<double>*)in, (cx<double>*)out, geom(c, p), mode);
+        k_adj_spectral<double><<<kRedBlocks, 256, 0, c->stream>>>((cx<double>*)w, (cx<double>*)kl,
+                                                                  (const cx<double>*)kpsi_np1, geom(c, p), c->red);
     else
-        k_adj_mul<float><<<g, 256, 0, c->stream>>>((const cx<float>*)in, (cx<float>*)out, geom(c, p), mode);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_adj_eps(const pfc_ctx* c, const void* lam_hat, const void* kpsi_np1, const pfc_step_params* p) {
-    if (c->dtype == PFC_F64)
-        k_adj_eps<double><<<kRedBlocks, 256, 0, c->stream>>>((const cx<double>*)lam_hat, (const cx<double>*)kpsi_np1,
-                                                             geom(c, p), c->red);
-    else
-        k_adj_eps<float><<<kRedBlocks, 256, 0, c->stream>>>((const cx<float>*)lam_hat, (const cx<float>*)kpsi_np1,
-                                                            geom(c, p), c->red);
+        k_adj_spectral<float><<<kRedBlocks, 256, 0, c->stream>>>((cx<float>*)w, (cx<float>*)kl,
+                                                                 (const cx<float>*)kpsi_np1, geom(c, p), c->red);
     cudaError_t e = cudaGetLastError();
-    if (e) return e;
+    if (e || !kpsi_np1) return e;
     return launch_reduce_final(c, 3, 1.0 / ((double)c->nx * c->ny * c->nz));
 }
 
@@ -169,10 +148,12 @@ cudaError_t launch_adj_combine(const pfc_ctx* c, void* lam, const void* psi_u, c
 cudaError_t launch_sf_loss(const pfc_ctx* c, const void* kpsi, const void* s_target, void* out) {
     if (c->dtype == PFC_F64)
         k_sf_loss<double><<<kRedBlocks, 256, 0, c->stream>>>((const cx<double>*)kpsi, (const double*)s_target,
-                                                             (cx<double>*)out, c->nx, c->ny, c->nz, c->red);
+                                                             (cx<double>*)out, c->nx, c->ny, c->nz,
+                                                            mode_index(c->nx, c->ny, c->nz), c->red);
     else
         k_sf_loss<float><<<kRedBlocks, 256, 0, c->stream>>>((const cx<float>*)kpsi, (const float*)s_target,
-                                                            (cx<float>*)out, c->nx, c->ny, c->nz, c->red);
+                                                            (cx<float>*)out, c->nx, c->ny, c->nz,
+                                                            mode_index(c->nx, c->ny, c->nz), c->red);
     cudaError_t e = cudaGetLastError();
     if (e) return e;
     return launch_reduce_final(c, 3, 1.0);

@@ -39,14 +39,14 @@ __device__ __forceinline__ float t_exp(float x) { return expf(x); }
 __device__ __forceinline__ double t_exp(double x) { return exp(x); }
 
 template <typename T>
-__global__ void k_gaussian_init(cx<T>* g, int nx, int ny, int nz, T lx, T ly, T lz, T hx, T hy, T hz, T dps) {
+__global__ void k_gaussian_init(cx<T>* g, int nx, int ny, int nz, T lx, T ly, T lz, T hx, T hy, T hz, T dps,
+                                ModeIndex mi) {
     const int nxh = nx / 2 + 1;
     const int64_t n = (int64_t)nxh * ny * nz;
     const T sx = T(1.1) * dps * hx, sy = T(1.1) * dps * hy, sz = T(1.1) * dps * hz;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
-        const int i0 = (int)(idx % nxh);
-        const int64_t r = idx / nxh;
-        const int i1 = (int)(r % ny), i2 = (int)(r / ny);
+        int i0, i1, i2;
+        mi.at(idx, i0, i1, i2);
         const T a = sx * kwave<T>(i0, nx, lx), b = sy * kwave<T>(i1, ny, ly), c = sz * kwave<T>(i2, nz, lz);
         const T e = t_exp(-T(0.5) * (a * a + b * b + c * c));
         g[idx] = cx<T>{e, T(1) - e};
@@ -174,12 +174,13 @@ bool write_gzip(const std::string& s, const char* path) {
 cudaError_t launch_gaussian_init(const pfc_ctx* c, void* g, double lx, double ly, double lz, double hx, double hy,
                                  double hz, double dps) {
     const int gs = grid_for(c->n_cmpl, 256);
+    const ModeIndex mi = mode_index(c->nx, c->ny, c->nz);
     if (c->dtype == PFC_F64)
         k_gaussian_init<double><<<gs, 256, 0, c->stream>>>((cx<double>*)g, c->nx, c->ny, c->nz, lx, ly, lz, hx, hy, hz,
-                                                           dps);
+                                                           dps, mi);
     else
         k_gaussian_init<float><<<gs, 256, 0, c->stream>>>((cx<float>*)g, c->nx, c->ny, c->nz, (float)lx, (float)ly,
-                                                          (float)lz, (float)hx, (float)hy, (float)hz, (float)dps);
+                                                          (float)lz, (float)hx, (float)hy, (float)hz, (float)dps, mi);
     return cudaGetLastError();
 }
 

@@ -20,15 +20,14 @@ template <typename T> __device__ __forceinline__ T ref_sqrtf(T x) { return (T)sq
 // stabilisation constant C (C = 1 is the reference: (1 + C - eps) = (2 - eps)).
 template <typename T>
 __global__ void k_update_eom(cx<T>* __restrict__ kpsi, const cx<T>* __restrict__ knl, cx<T>* knoise, int nx, int ny,
-                             int nz, T namp_eff, T dt, T eps, T lx, T ly, T lz, int with_fen, T C) {
+                             int nz, T namp_eff, T dt, T eps, T lx, T ly, T lz, int with_fen, T C, ModeIndex mi) {
     const int nxh = nx / 2 + 1;
     const int64_t total = (int64_t)nxh * ny * nz;
     const T deps = T(1) + C - eps;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        const int i0 = (int)(idx % nxh);
-        const int64_t r = idx / nxh;
-        const int i1 = (int)(r % ny), i2 = (int)(r / ny);
+        int i0, i1, i2;
+        mi.at(idx, i0, i1, i2);
         const cx<T> p = kpsi[idx];
         const cx<T> q = knl[idx];
         const cx<T> w = knoise ? knoise[idx] : mkc<T>(T(0), T(0));
@@ -101,19 +100,20 @@ __global__ void __launch_bounds__(256) k_calc_fen(const T* __restrict__ psi, T* 
 }
 
 // sum over the half spectrum of w_k |psi^_k|^2 (L^_k - 1), w_k = 2 for 0 < i0 < nx/2
-// (Parseval: sum_x psi (L-1) psi = (1/N) sum_k |psi^_k|^2 (L^_k - 1) over the full grid).
+// (Parseval: sum_x psi (L-1) psi = (1/N) sum_k |psi^_k|^2 (L^_k - 1) over the full grid).  ck =
+// 2 pi / L per axis: three FP64 divisions per mode made the kernel FP64-bound.
 template <typename T>
 __global__ void __launch_bounds__(256) k_fen_spectral(const cx<T>* __restrict__ kpsi, int nx, int ny, int nz, double eps,
-                                                      double lx, double ly, double lz, double* __restrict__ partial) {
+                                                      double ckx, double cky, double ckz, ModeIndex mi,
+                                                      double* __restrict__ partial) {
     const int nxh = nx / 2 + 1;
     const int64_t total = (int64_t)nxh * ny * nz;
     double s = 0.0, c = 0.0;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        const int i0 = (int)(idx % nxh);
-        const int64_t r = idx / nxh;
-        const int i1 = (int)(r % ny), i2 = (int)(r / ny);
-        const double k0 = kwave<double>(i0, nx, lx), k1 = kwave<double>(i1, ny, ly), k2 = kwave<double>(i2, nz, lz);
+        int i0, i1, i2;
+        mi.at(idx, i0, i1, i2);
+        const double k0 = kwave_ck<double>(i0, nx, ckx), k1 = kwave_ck<double>(i1, ny, cky), k2 = kwave_ck<double>(i2, nz, ckz);
         const double k2s = k0 * k0 + k1 * k1 + k2 * k2;
         const double lm1 = (1.0 - eps) - 2.0 * k2s + k2s * k2s;
         const double w = (i0 == 0 || (((nx & 1) == 0) && i0 == nx / 2)) ? 1.0 : 2.0;
@@ -151,14 +151,15 @@ __global__ void k_reduce_final(const double* __restrict__ partial, int nb, doubl
 }
 
 template <typename T>
-__global__ void k_noise_kspace(cx<T>* __restrict__ arr, int nx, int ny, int nz, uint64_t seed, uint64_t counter) {
+__global__ void k_noise_kspace(cx<T>* __restrict__ arr, int nx, int ny, int nz, uint64_t seed, uint64_t counter,
+                               ModeIndex mi) {
     const int nxh = nx / 2 + 1;
     const int64_t total = (int64_t)nxh * ny * nz;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        const int i0 = (int)(idx % nxh);
-        const int64_t r = idx / nxh;
-        arr[idx] = kspace_noise<T>(i0, (int)(r % ny), (int)(r / ny), nx, ny, nz, seed, counter);
+        int i0, i1, i2;
+        mi.at(idx, i0, i1, i2);
+        arr[idx] = kspace_noise<T>(i0, i1, i2, nx, ny, nz, seed, counter);
     }
 }
 
@@ -204,16 +205,17 @@ cudaError_t launch_counter(cudaStream_t st, unsigned long long* ctr, unsigned lo
 cudaError_t launch_update_eom(const pfc_ctx* c, void* kpsi, const void* knl, const void* knoise, double namp,
                               double dt, double eps, double lx, double ly, double lz, int with_fen, double C) {
     const int g = grid_for(c->n_cmpl, 256);
+    const ModeIndex mi = mode_index(c->nx, c->ny, c->nz);
     if (c->dtype == PFC_F64) {
         // reference: namp *= sqrtf(nx*ny*nz)  (eom.hpp:62)
         const double ne = namp * (double)sqrtf((float)(c->nx * c->ny * c->nz));
         k_update_eom<double><<<g, 256, 0, c->stream>>>((cx<double>*)kpsi, (const cx<double>*)knl, (cx<double>*)knoise,
-                                                        c->nx, c->ny, c->nz, ne, dt, eps, lx, ly, lz, with_fen, C);
+                                                        c->nx, c->ny, c->nz, ne, dt, eps, lx, ly, lz, with_fen, C, mi);
     } else {
         const float ne = (float)namp * sqrtf((float)(c->nx * c->ny * c->nz));
         k_update_eom<float><<<g, 256, 0, c->stream>>>((cx<float>*)kpsi, (const cx<float>*)knl, (cx<float>*)knoise,
                                                        c->nx, c->ny, c->nz, ne, (float)dt, (float)eps, (float)lx,
-                                                       (float)ly, (float)lz, with_fen, (float)C);
+                                                       (float)ly, (float)lz, with_fen, (float)C, mi);
     }
     return cudaGetLastError();
 }
@@ -256,12 +258,14 @@ cudaError_t launch_calc_fen(const pfc_ctx* c, const void* psi, void* lpsi, doubl
 }
 
 cudaError_t launch_fen_spectral(const pfc_ctx* c, const void* kpsi, double eps, double lx, double ly, double lz) {
+    const double tp = 6.283185307179586232, cx_ = tp / lx, cy = tp / ly, cz = tp / lz;
+    const ModeIndex mi = mode_index(c->nx, c->ny, c->nz);
     if (c->dtype == PFC_F64)
         k_fen_spectral<double><<<kRedBlocks, 256, 0, c->stream>>>((const cx<double>*)kpsi, c->nx, c->ny, c->nz, eps,
-                                                                   lx, ly, lz, c->red);
+                                                                   cx_, cy, cz, mi, c->red);
     else
-        k_fen_spectral<float><<<kRedBlocks, 256, 0, c->stream>>>((const cx<float>*)kpsi, c->nx, c->ny, c->nz, eps, lx,
-                                                                  ly, lz, c->red);
+        k_fen_spectral<float><<<kRedBlocks, 256, 0, c->stream>>>((const cx<float>*)kpsi, c->nx, c->ny, c->nz, eps, cx_,
+                                                                  cy, cz, mi, c->red);
     return cudaGetLastError();
 }
 
@@ -274,10 +278,11 @@ cudaError_t launch_quartic_sum(const pfc_ctx* c, const void* v, double mul) {
 
 cudaError_t launch_noise_kspace(const pfc_ctx* c, void* arr, uint64_t seed, uint64_t counter) {
     const int g = grid_for(c->n_cmpl, 256);
+    const ModeIndex mi = mode_index(c->nx, c->ny, c->nz);
     if (c->dtype == PFC_F64)
-        k_noise_kspace<double><<<g, 256, 0, c->stream>>>((cx<double>*)arr, c->nx, c->ny, c->nz, seed, counter);
+        k_noise_kspace<double><<<g, 256, 0, c->stream>>>((cx<double>*)arr, c->nx, c->ny, c->nz, seed, counter, mi);
     else
-        k_noise_kspace<float><<<g, 256, 0, c->stream>>>((cx<float>*)arr, c->nx, c->ny, c->nz, seed, counter);
+        k_noise_kspace<float><<<g, 256, 0, c->stream>>>((cx<float>*)arr, c->nx, c->ny, c->nz, seed, counter, mi);
     return cudaGetLastError();
 }
 

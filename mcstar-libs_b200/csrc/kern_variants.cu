@@ -31,14 +31,9 @@ template <typename T> __device__ __forceinline__ T f_exp(T x) { return (T)expf((
 
 struct Modes {
     int nx, ny, nz;
+    ModeIndex mi;
     __device__ __forceinline__ int64_t total() const { return (int64_t)(nx / 2 + 1) * ny * nz; }
-    __device__ __forceinline__ void at(int64_t idx, int& i0, int& i1, int& i2) const {
-        const int nxh = nx / 2 + 1;
-        i0 = (int)(idx % nxh);
-        const int64_t r = idx / nxh;
-        i1 = (int)(r % ny);
-        i2 = (int)(r / ny);
-    }
+    __device__ __forceinline__ void at(int64_t idx, int& i0, int& i1, int& i2) const { mi.at(idx, i0, i1, i2); }
 };
 
 // dop = (-k^2, k^4) of L_L2 (common.hpp:17-22) with K (common.hpp:27-28)
@@ -185,7 +180,7 @@ __global__ void k_update_eom_hpfcnoise(cx<T>* kpsi, const cx<T>* __restrict__ kn
     }
 }
 
-Modes modes(const pfc_ctx* c) { return Modes{c->nx, c->ny, c->nz}; }
+Modes modes(const pfc_ctx* c) { return Modes{c->nx, c->ny, c->nz, mode_index(c->nx, c->ny, c->nz)}; }
 
 // the reference's namp *= sqrtf(nx*ny*nz), in the field's precision
 double namp_scaled(const pfc_ctx* c, double namp) {

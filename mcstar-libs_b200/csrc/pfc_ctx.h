@@ -256,8 +256,8 @@ cudaError_t launch_update_eom_hpfcnoise(const pfc_ctx* c, void* kpsi, const void
                                         double lz);
 
 // ---- adjoint of the step (kern_adjoint.cu); the sums land in red slot 3 ----
-cudaError_t launch_adj_mul(const pfc_ctx* c, const void* in, void* out, const pfc_step_params* p, int mode);
-cudaError_t launch_adj_eps(const pfc_ctx* c, const void* lam_hat, const void* kpsi_np1, const pfc_step_params* p);
+// w = lam^ -> lam^ / D over it and (dt k^2 / D) lam^ into kl; kpsi_np1 (or null): the eps sum
+cudaError_t launch_adj_spectral(const pfc_ctx* c, void* w, void* kl, const void* kpsi_np1, const pfc_step_params* p);
 cudaError_t launch_adj_combine(const pfc_ctx* c, void* lam, const void* psi_u, const void* b, double C);
 cudaError_t launch_sf_loss(const pfc_ctx* c, const void* kpsi, const void* s_target, void* out);
 
