@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 #include "bulk.cuh"
+#include "chain.cuh"
 #include "genpass.cuh"
 #include "pfc_ctx.h"
 
@@ -776,6 +777,7 @@ size_t pfc_workspace_bytes(const pfc_ctx* ctx) {
 pfc_status pfc_fft_r2c(pfc_ctx* ctx, const void* in, void* out) {
     PFC_CHECK_CTX();
     if (!in || !out) return fail(ctx, PFC_ERR_INVALID, "pfc_fft_r2c: null buffer");
+    const ChainScope chained(ctx);
     const bool reg_xy = ctx->fused_x && ctx->fused_y;
     if (reg_xy) PFC_CUDA(launch_xrows_r2c(ctx, in, out), "pfc_fft_r2c rows");
     else PFC_CUDA(launch_rows_r2c(ctx, in, out), "pfc_fft_r2c rows");
@@ -788,6 +790,7 @@ pfc_status pfc_fft_r2c(pfc_ctx* ctx, const void* in, void* out) {
 pfc_status pfc_fft_c2r(pfc_ctx* ctx, const void* in, void* out) {
     PFC_CHECK_CTX();
     if (!in || !out) return fail(ctx, PFC_ERR_INVALID, "pfc_fft_c2r: null buffer");
+    const ChainScope chained(ctx);
     const void* src = in;  // the input is left unchanged: the passes run in the workspace
     if (ctx->nz > 1) { PFC_CUDA(zcols(ctx, 1, src, ctx->work, 1.0), "pfc_fft_c2r z"); src = ctx->work; }
     if (ctx->ny > 1) { PFC_CUDA(ycols(ctx, 1, src, ctx->work), "pfc_fft_c2r y"); src = ctx->work; }
@@ -972,6 +975,7 @@ pfc_status pfc_step_prop(pfc_ctx* ctx, void* kpsi, int nsteps, const pfc_step_pa
         return fail(ctx, PFC_ERR_INVALID, "pfc_step_prop: the relaxation propagators take no noise (el.hpp)");
     if (max_change) *max_change = 0.0;
     if (nsteps == 0) return PFC_OK;
+    const ChainScope chained(ctx);
     ZPropArgs za = zargs(ctx, p);
     za.prop = propagator;
     // flag[0]: the watchdog and wait status; flag[2]: the last step's largest mode change

@@ -1,6 +1,7 @@
 // The general column and row passes (genpass.cuh): kernels and launchers, instantiated per
 // precision by kern_gen32.cu and kern_gen64.cu.
 #pragma once
+#include "chain.cuh"
 #include "genpass.cuh"
 
 namespace pfc {
@@ -19,6 +20,8 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
            const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, double scale, int64_t ms) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
+    chain_start();
+    chain_wait();
     const ColLines lay{lg};
     const ColTile<T> tile{lg, ni};
     const int64_t base = (int64_t)blockIdx.y * os + tile.i0 + blockIdx.z * ms;  // grid z: fields of a batch
@@ -92,6 +95,8 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
            double mul, double C, double mu, int64_t ms, FastDiv by_nxh) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
+    chain_start();
+    chain_wait();
     constexpr int W = Elem<T>::lines;
     const int row0 = blockIdx.x * rpc * W;
     const int nr = min(rpc * W, nrows - row0), nl = (nr + W - 1) / W;
@@ -224,9 +229,8 @@ cudaError_t gen_cols(const pfc_ctx* c, int axis, int dir, const void* in, void* 
     const int tile = Elem<T>::lines << ap.lg;
     dim3 grid((c->nxh + tile - 1) / tile, no, c->batch);
     auto k = dir < 0 ? k_cols<T, -1> : k_cols<T, 1>;
-    k<<<grid, ap.threads, ap.smem, c->stream>>>((const cx<T>*)in, (cx<T>*)out, c->nxh, es, os, ap.plan,
-                                                (const el<T>*)c->gtw, c->fft_tab, ap.lg, scale, c->mstride);
-    return cudaGetLastError();
+    return chain_launch(c, k, grid, ap.threads, ap.smem, (const cx<T>*)in, (cx<T>*)out, c->nxh, es, os, ap.plan,
+                        (const el<T>*)c->gtw, c->fft_tab, ap.lg, scale, c->mstride);
 }
 
 template <typename T>
@@ -238,8 +242,7 @@ cudaError_t gen_rows(const pfc_ctx* c, int mode, const void* in, void* out, doub
     // (the plain transforms run on one field; the x pass on all fields of a batch)
     dim3 grid((nrows + rows - 1) / rows, 1, mode == kNonlin ? c->batch : 1);
     auto k = mode == kR2C ? k_rows<T, kR2C> : mode == kC2R ? k_rows<T, kC2R> : k_rows<T, kNonlin>;
-    k<<<grid, ap.threads, ap.smem, c->stream>>>(in, out, nrows, c->nx, ap.plan, tw, c->fft_tab, tw + c->post_off,
-                                                ap.lines, mul, C, mu, c->mstride, make_fastdiv(c->nxh));
-    return cudaGetLastError();
+    return chain_launch(c, k, grid, ap.threads, ap.smem, in, out, nrows, c->nx, ap.plan, tw, c->fft_tab,
+                        tw + c->post_off, ap.lines, mul, C, mu, c->mstride, make_fastdiv(c->nxh));
 }
 }  // namespace pfc

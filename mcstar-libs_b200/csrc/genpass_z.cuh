@@ -1,6 +1,7 @@
 // The general z pass of the stepper (genpass.cuh): kernel and launcher, instantiated per
 // precision by kern_genz32.cu and kern_genz64.cu.
 #pragma once
+#include "chain.cuh"
 #include "genpass.cuh"
 
 namespace pfc {
@@ -66,8 +67,8 @@ __device__ __forceinline__ cx<T> zmode_of(cx<T> psi, cx<T> nl, const ZColumn<T>&
         const T f = a.dt * dopx;
         cx<T> num = mkc<T>(psi.x + f * nl.x, psi.y + f * nl.y);
         if (a.use_noise) {
-            const cx<T> xi = kspace_noise<T>(kx, kyg, kz, nx, a.nyg, nz, a.seed, a.counter, kKspaceDomain, -dopx);
-            const T g = a.dt * a.namp_eff;
+            const cx<T> xi = kspace_noise<T>(kx, kyg, kz, nx, a.nyg, nz, a.seed, a.counter);
+            const T g = a.dt * a.namp_eff * sqrt(-dopx);
             num.x += g * xi.x;
             num.y += g * xi.y;
         }
@@ -119,6 +120,8 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
             cx<T>* anext) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
+    chain_start();
+    chain_wait();
     zmember(a);
     const int nxh = nx / 2 + 1, n = p.n;
     const ColTile<T> tile{lg, nxh};
@@ -227,10 +230,9 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
                 (T)(tp / (flat ? a.ly : a.lz)), a.seed, a.counter, a.dev_counter, a.use_noise, a.final_step, a.prop,
                 a.maxc, a.margs, a.ky0, a.ny_global > 0 ? a.ny_global : ny};
     auto k = carry ? k_zprop<T, true> : k_zprop<T, false>;
-    k<<<grid, ap.threads, carry ? ap.smem : 2 * ap.smem, c->stream>>>(
-        (cx<T>*)A, (const cx<T>*)B, c->nx, ny, ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, t, c->k0, c->flag,
-        c->mstride, (cx<T>*)anext);
-    return cudaGetLastError();
+    return chain_launch(c, k, grid, ap.threads, carry ? ap.smem : 2 * ap.smem, (cx<T>*)A, (const cx<T>*)B, c->nx, ny,
+                        ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, t, c->k0, c->flag, c->mstride,
+                        (cx<T>*)anext);
 }
 
 }  // namespace pfc

@@ -14,6 +14,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include "bulk.cuh"
+#include "chain.cuh"
 #include "pfc_ctx.h"
 #include "regfft.cuh"
 
@@ -56,7 +57,9 @@ __global__ void __launch_bounds__(Y::T, Y::MINB)
     float2* xb = sm;
     float2* tw = sm + Y::XB;
     const int tid = threadIdx.x;
+    chain_start();
     for (int i = tid; i < NY; i += Y::T) tw[i] = twg[i];
+    chain_wait();
     const int c = tid % TX, t = tid / TX;
     const int kx = blockIdx.x * TX + c;
     const bool valid = kx < nxh;
@@ -336,7 +339,9 @@ __global__ void __launch_bounds__(X::T, X::MINB)
     float2* twM = sm + X::BUF;  // W_M^m, m < M
     float2* twP = twM + M;      // W_NX^k, k <= M
     const int tid = threadIdx.x;
+    chain_start();
     for (int i = tid; i < 2 * M + 1; i += X::T) twM[i] = twg[i];
+    chain_wait();
     const int r = tid % R, t = tid / R;
     const int row0 = blockIdx.x * R;
     const int nr = min(R, nrows - row0);
@@ -775,13 +780,9 @@ cudaError_t collaunch(const pfc_ctx* c, int dir, const void* in, void* out, doub
                       int tw_off, int q0 = 0, void* copy = nullptr) {
     dim3 grid((c->nxh + Y::TX - 1) / Y::TX, planes, c->batch);
     const float2* tw = reinterpret_cast<const float2*>(c->tw) + tw_off;
-    if (dir > 0)
-        k_ycol<Y, 1, kZ><<<grid, Y::T, Y::SMEM, c->stream>>>((const float2*)in, (float2*)out, c->nxh, c->ny, c->nz,
-                                                             lay, tw, (float)scale, c->mstride, q0, (float2*)copy);
-    else
-        k_ycol<Y, -1, kZ><<<grid, Y::T, Y::SMEM, c->stream>>>((const float2*)in, (float2*)out, c->nxh, c->ny, c->nz,
-                                                              lay, tw, (float)scale, c->mstride, q0, (float2*)copy);
-    return cudaGetLastError();
+    auto k = dir > 0 ? k_ycol<Y, 1, kZ> : k_ycol<Y, -1, kZ>;
+    return chain_launch(c, k, grid, Y::T, Y::SMEM, (const float2*)in, (float2*)out, c->nxh, c->ny, c->nz, lay, tw,
+                        (float)scale, c->mstride, q0, (float2*)copy);
 }
 template <class Y>
 cudaError_t ylaunch(const pfc_ctx* c, int dir, const void* in, void* out, double scale, int nzs, int lay) {
@@ -799,9 +800,8 @@ cudaError_t xlaunch(const pfc_ctx* c, const void* in, void* out, const void* pot
     const float2* tw = reinterpret_cast<const float2*>(c->tw) + c->xpass_tw_off;
     if (MODE == 3 && nrows % X::R) return cudaErrorNotSupported;  // whole tiles of rows
     if (pot && c->batch > 1) return cudaErrorNotSupported;
-    k_xrow<X, MODE><<<grid, X::T, X::SMEM, c->stream>>>((const float2*)in, (float2*)out, (const float*)pot, nrows, tw,
-                                                        (float)mul, (float)C, (float)mu, c->mstride);
-    return cudaGetLastError();
+    return chain_launch(c, k_xrow<X, MODE>, grid, X::T, X::SMEM, (const float2*)in, (float2*)out, (const float*)pot,
+                        nrows, tw, (float)mul, (float)C, (float)mu, c->mstride);
 }
 
 }  // namespace

@@ -81,6 +81,7 @@ struct pfc_ctx {
     int ykern;                    // the y pass between the tiled layouts: 0 k_ycol3, 1 k_ybulk (TMA)
     int xpair_tw_off;             // W_nx^m, m < nx
     int xy_mode;                  // 0 general passes, 2 register y/x/y passes
+    bool chain = false;           // launches of the call in progress are chained (chain.cuh)
     // tracing (pfc_profile_enable / pfc_profile_read)
     bool prof_on = false;
     long long launches = 0;

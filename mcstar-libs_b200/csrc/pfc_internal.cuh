@@ -313,62 +313,58 @@ __device__ __forceinline__ void cos_sin_2pi(uint64_t m, double& co, double& si) 
     si = (q & 2) ? -y : y;
 }
 
-// sqrt(-v log u1) (cos, sin)(2 pi u2) from counter (idx, counter) under key (seed, domain),
-// u1 and u2 uniform strictly inside (0, 1) and exact in T (Box-Muller; v = 2 gives two
-// standard normals).
-template <typename T> __device__ __forceinline__ cx<T> philox_polar(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                    uint32_t domain, T v);
-template <> __device__ __forceinline__ float2 philox_polar<float>(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                  uint32_t domain, float v) {
-    const U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
-    const U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
+// Two standard normals from counter (idx, counter) under key (seed, domain),
+// Box-Muller on uniforms strictly inside (0, 1) that are exact in T.
+template <typename T> __device__ __forceinline__ void philox_normal2(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                     uint32_t domain, T& g1, T& g2);
+template <> __device__ __forceinline__ void philox_normal2<float>(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                  uint32_t domain, float& g1, float& g2) {
+    U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
+    U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
     const float u1 = (float)((r.x >> 9) * 2u + 1u) * 5.9604644775390625e-08f;  // 2^-24
-    const float rad = sqrtf(-v * logf(u1));
     const float u2 = (float)((r.y >> 9) * 2u + 1u) * 5.9604644775390625e-08f;
+    const float rad = sqrtf(-2.0f * logf(u1));
     float s, co;
     sincospif(2.0f * u2, &s, &co);
-    return make_float2(rad * co, rad * s);
+    g1 = rad * co; g2 = rad * s;
 }
-template <> __device__ __forceinline__ double2 philox_polar<double>(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                    uint32_t domain, double v) {
-    const U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
-    const U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
+template <> __device__ __forceinline__ void philox_normal2<double>(uint64_t idx, uint64_t seed, uint64_t counter,
+                                                                   uint32_t domain, double& g1, double& g2) {
+    U4 c{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)counter, (uint32_t)(counter >> 32)};
+    U4 r = philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32) ^ domain);
     const uint64_t a = ((((uint64_t)r.x << 32) | r.y) >> 12) * 2u + 1u;
     const uint64_t b = ((((uint64_t)r.z << 32) | r.w) >> 12) * 2u + 1u;
     const double u1 = (double)a * 1.1102230246251565404e-16;  // 2^-53
-    const double rad = sqrt(-v * log(u1));
+    const double rad = sqrt(-2.0 * log(u1));
     double s, co;
     cos_sin_2pi(b, co, s);
-    return make_double2(rad * co, rad * s);
-}
-template <typename T> __device__ __forceinline__ void philox_normal2(uint64_t idx, uint64_t seed, uint64_t counter,
-                                                                     uint32_t domain, T& g1, T& g2) {
-    const cx<T> g = philox_polar<T>(idx, seed, counter, domain, T(2));
-    g1 = g.x;
-    g2 = g.y;
+    g1 = rad * co; g2 = rad * s;
 }
 
-// sqrt(v) times the k-space noise of half-spectrum mode (i0, i1, i2): complex normal with unit
-// variance; modes on the i0 = 0 and i0 = nx/2 planes are keyed by the canonical (lower linear
-// index) member of their +-k pair and conjugated on the other member; self-conjugate modes
-// are real.  (v = k^2 gives the conserved noise |k| xi with one square root.)
+// k-space noise of half-spectrum mode (i0, i1, i2): modes on the i0 = 0 and
+// i0 = nx/2 planes are keyed by the canonical (lower linear index) member of their
+// +-k pair and conjugated on the other member; self-conjugate modes are real.
 template <typename T>
 __device__ __forceinline__ cx<T> kspace_noise(int i0, int i1, int i2, int nx, int ny, int nz, uint64_t seed,
-                                              uint64_t counter, uint32_t domain = kKspaceDomain, T v = T(1)) {
+                                              uint64_t counter, uint32_t domain = kKspaceDomain) {
     const int nxh = nx / 2 + 1, plane = ny * nxh;  // (a plane's modes fit an int: lengths are at most some 10^4)
     int64_t key = (int64_t)i2 * plane + (i1 * nxh + i0);
-    T fy = T(1);  // -1 on the conjugate member, 0 on a self-conjugate mode
+    const T h = T(0.70710678118654752440);
+    T fx = h, fy = h;
     if (i0 == 0 || 2 * i0 == nx) {
         const int j1 = i1 == 0 ? 0 : ny - i1;
         const int j2 = i2 == 0 ? 0 : nz - i2;
         const int64_t part = (int64_t)j2 * plane + (j1 * nxh + i0);
-        if (part <= key) fy = part < key ? T(-1) : T(0);
-        if (part == key) v = v * T(2);
+        if (part < key) fy = -h;
+        if (part == key) {
+            fx = T(1);
+            fy = T(0);
+        }
         key = min(key, part);
     }
-    cx<T> g = philox_polar<T>((uint64_t)key, seed, counter, domain, v);
-    g.y *= fy;
-    return g;
+    T g1, g2;
+    philox_normal2<T>((uint64_t)key, seed, counter, domain, g1, g2);
+    return mkc<T>(g1 * fx, g2 * fy);
 }
 
 // The anisotropic 2D noise of eom.hpp:16-58 at wavenumbers (k0, k1), |k| = kabs: the three

@@ -225,6 +225,21 @@ __device__ __forceinline__ ColAddr zcol_addr(int kt, int c, int ky, int nxh, int
     return ColAddr{((int64_t)kt * kTileW * ny + ky * wt) * nz + c, (int64_t)wt};
 }
 
+// The last kx tile of nxh = nx/2 + 1 columns holds kx = nx/2 alone when 8 divides nx/2: as a tile
+// of its own it would do the work of TX columns for one (13 tiles for 97 columns).  Its CTAs take
+// that column at TX consecutive ky instead, ky = TX blockIdx.y + c, and the rest of the tile's
+// CTAs leave.  False: this CTA leaves.  Tiles of several columns, and row counts TX does not
+// divide, stay as they are.  (Z pass carrying A, FP32 with noise: 192^3 step 111.0 -> 106.2 us,
+// 256^3 235.6 -> 229.7.  In the y passes the per-lane plane index cost more than the work saved.)
+template <int TX>
+__device__ __forceinline__ bool edge_tile(int kt, int nxh, int planes, int c, int& kx, int& q) {
+    if (nxh % TX != 1 || kt != nxh / TX || planes % TX) return true;
+    if (q >= planes / TX) return false;
+    kx = nxh - 1;
+    q = q * TX + c;
+    return true;
+}
+
 // Exchange slots: group g of NG interleaved groups, logical index (a, b) of an
 // E x P matrix -> (a P + b) NG + a PADG + g.  Warps run over consecutive g (and, when
 // NG < 32, over 32/NG consecutive t); PADG shifts successive blocks of P rows so that

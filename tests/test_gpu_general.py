@@ -65,3 +65,19 @@ def test_general_steps_and_resume(shape, dtype):
     assert rel(runs[0], want) < (2e-6 if dtype == F32 else 1e-12)
     assert np.array_equal(runs[0], runs[1])
     assert runs[0][0, 0, 0] == k0.astype(runs[0].dtype)[0, 0, 0]
+
+
+@pytest.mark.parametrize("shape", [(16, 16, 256), (16, 12, 256), (32, 8, 128), (48, 24, 192), (64, 64, 128)], ids=str)
+def test_edge_column_tiles(shape):
+    """The register z pass whose last tile is the kx = nx/2 column alone takes it at eight ky per
+    CTA where 8 divides ny, and as a tile of its own elsewhere (ny = 12)."""
+    from mcstar_b200 import Stepper
+    nx, ny, nz = shape
+    k0 = O.r2c(-0.2 + 0.1 * np.random.default_rng(9).uniform(-1, 1, (nz, ny, nx)))
+    st = Stepper(shape, math.pi / 4, 0.5, 0.3, dtype=F32, namp=0.03, seed=3)
+    st.set_kspace(k0.astype(np.complex64))
+    st.step(4)
+    want = O.step(k0, 4, 0.5, 0.3, st.lens, shape, namp=0.03, seed=3, noise_dtype=F32)
+    got = st.kspace()
+    assert rel(got, want) < 2e-6
+    assert rel(got[..., nx // 2], want[..., nx // 2]) < 2e-5
