@@ -23,6 +23,8 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
 // 240 x 200 x 180 FP32 took 0.025 / 0.049 / 0.088 ms (y, x, z) against 0.021 / 0.044 / 0.060.
 template <typename T> constexpr int kGenCtas = sizeof(T) == 8 ? 3 : 4;
 constexpr int kGenThreads = 256;
+// largest first radix of the stepper's paired x pass (two butterflies in registers)
+constexpr int kPairRadix = 5;
 
 // The columns of a CTA: 2^lg elements of one column (FP64) or of two columns 2^lg apart (FP32;
 // consecutive threads then move consecutive columns of either half), from column i0 of ni.

@@ -37,6 +37,7 @@ struct pfc_ctx {
     pfc_options opt;              // the options in effect (pfc_get_options)
 
     pfc::AxisPlan px;             // x: complex length nx/2 (even nx) or nx (odd nx)
+    pfc::AxisPlan px2;            // the stepper's x pass (even nx): first radix at most kPairRadix (nst 0: none)
     pfc::AxisPlan py, pz;         // y, z: complex length ny, nz
     pfc::AxisPlan pzprop, pz2;    // the stepper's z pass carrying psi^; carrying A (two lines per column)
     pfc::AxisPlan py2;            // the stepper's update pass along the y columns of a 2D field

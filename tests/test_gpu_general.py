@@ -81,3 +81,20 @@ def test_edge_column_tiles(shape):
     got = st.kspace()
     assert rel(got, want) < 2e-6
     assert rel(got[..., nx // 2], want[..., nx // 2]) < 2e-5
+
+
+@pytest.mark.parametrize("dtype", [F32, F64], ids=["f32", "f64"])
+@pytest.mark.parametrize("shape", [(4, 4, 1), (8, 6, 5), (10, 3, 1), (36, 5, 1), (54, 7, 3), (50, 11, 2), (90, 9, 1),
+                                   (72, 30, 4), (2400, 3, 1)], ids=str)
+def test_paired_x_pass(shape, dtype):
+    """The x pass that splits and merges the real transforms in the first stage's registers: first
+    radices 2 to 5, odd and even numbers of its butterflies (the middle one pairs with itself),
+    an appended stage of radix 1, an unpaired last row in FP32."""
+    from mcstar_b200 import Stepper
+    nx, ny, nz = shape
+    k0 = O.r2c(-0.2 + 0.1 * np.random.default_rng(4).uniform(-1, 1, (nz, ny, nx)))
+    st = Stepper(shape, math.pi / 4, 0.25, 0.3, dtype=dtype)
+    st.set_kspace(k0.astype(np.complex64 if dtype == F32 else np.complex128))
+    st.step(3)
+    want = O.step(k0, 3, 0.25, 0.3, st.lens, shape)
+    assert rel(st.kspace(), want) < (2e-6 if dtype == F32 else 1e-12)
