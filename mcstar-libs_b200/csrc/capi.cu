@@ -666,11 +666,12 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     // 16 FP32 or 8 FP64 columns), halved down to the 32-byte sectors of L2 while the tile's
     // shared memory would leave fewer than three CTAs per SM, or the pass fewer than two CTAs
     // per SM; then tile_shift times.  Threads: one butterfly each in the stage with the most, up
-    // to 256 (FP64: 128, for more CTAs per SM, unless the pass has too few CTAs for that).
+    // to 256 (FP64: 128, for more CTAs per SM, unless the pass has too few CTAs for that); the
+    // update passes with few CTAs take one mode each, the update being their longest part.
     // Rows: as many as fill those threads.
     const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
     const int many = c->dtype == PFC_F64 ? 128 : 256;
-    auto columns = [&](AxisPlan& ap, int64_t planes, int fields, int shift) {
+    auto columns = [&](AxisPlan& ap, int64_t planes, int fields, bool update, int shift) {
         const size_t line = (size_t)ap.plan.np * 16 * fields;
         int lg = 3;
         auto ctas = [&] { return ((c->nxh + (W << lg) - 1) / (W << lg)) * planes; };
@@ -678,15 +679,16 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
         while (lg > 0 && (line << lg) > kMaxDynSmem) --lg;
         lg = std::max(0, lg - shift);
         ap.lg = lg;
-        const int most = ctas() < 4 * (int64_t)c->num_sms ? kGenThreads : many;
-        ap.threads = std::min(most, std::max(32, ((ap.plan.nbmax * fields << lg) + 31) & ~31));
+        const bool few = ctas() < 4 * (int64_t)c->num_sms;
+        const int work = ((few && update ? ap.plan.n : ap.plan.nbmax * fields) << lg) + 31;
+        ap.threads = std::min(few ? kGenThreads : many, std::max(32, work & ~31));
         ap.smem = ((size_t)ap.plan.np * 16) << lg;
     };
-    columns(c->py, c->nz, 1, o.tile_shift[1]);
-    columns(c->pz, c->ny, 1, o.tile_shift[2]);
-    columns(c->pzprop, c->ny, 1, o.tile_shift[3]);
-    columns(c->pz2, c->ny, 2, o.tile_shift[3]);
-    columns(c->py2, 1, 1, o.tile_shift[3]);
+    columns(c->py, c->nz, 1, false, o.tile_shift[1]);
+    columns(c->pz, c->ny, 1, false, o.tile_shift[2]);
+    columns(c->pzprop, c->ny, 1, true, o.tile_shift[3]);
+    columns(c->pz2, c->ny, 2, true, o.tile_shift[3]);
+    columns(c->py2, 1, 1, true, o.tile_shift[3]);
     auto rows = [&](AxisPlan& ap, int work) {  // work: the most items of a line in a stage
         const int64_t nrows = (int64_t)c->ny * c->nz;
         int lines = std::max(1, many / work);
