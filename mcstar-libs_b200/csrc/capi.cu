@@ -139,6 +139,58 @@ bool make_plan(int n, GPlan& p, std::vector<std::complex<double>>& tab, std::vec
     return true;
 }
 
+// Lines per CTA and threads of the general passes for `batch` fields on `sms` multiprocessors (a
+// class of an ensemble shares the GPU with the other classes).
+void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) {
+    // Columns: 128-byte segments (8 elements of 16 bytes:
+    // 16 FP32 or 8 FP64 columns), halved down to the 32-byte sectors of L2 while the tile's
+    // shared memory would leave fewer than three CTAs per SM, or the pass fewer than two CTAs
+    // per SM; then tile_shift times.  Threads: one butterfly each in the stage with the most, up
+    // to 256 (FP64: 128, for more CTAs per SM); a pass with at most four CTAs per SM takes 256, with
+    // at most two the SM's whole register file, and an update pass with few CTAs one mode per
+    // thread: the update is its longest part (1000^2 FP32 step, 126 CTAs: 46.3 us at 256 threads,
+    // 28.3 at 1000; with noise 59.6 and 31.7; two-column tiles at 256 threads 33.4 and 34.0).
+    // Rows: as many as fill those threads.
+    const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
+    const int many = c->dtype == PFC_F64 ? 128 : 256;
+    auto columns = [&](AxisPlan& ap, int64_t planes, int fields, bool update, int shift) {
+        const size_t line = (size_t)ap.plan.np * 16 * fields;
+        int lg = 3;
+        auto ctas = [&] { return ((c->nxh + (W << lg) - 1) / (W << lg)) * planes * batch; };
+        while (lg > 1 && ((line << lg) > 72 * 1024 || ctas() < 2 * (int64_t)sms)) --lg;
+        while (lg > 0 && (line << lg) > kMaxDynSmem) --lg;
+        lg = std::max(0, lg - shift);
+        ap.lg = lg;
+        const int64_t per_sm = (ctas() + sms - 1) / sms;
+        const bool few = per_sm <= 4;
+        const int work = ((few && update ? ap.plan.n : ap.plan.nbmax * fields) << lg) + 31;
+        const int full = c->dtype == PFC_F64 ? kColThreads<double> : kColThreads<float>;
+        const int most = !few ? many : per_sm <= 2 ? (int)(full / per_sm) & ~31 : kGenThreads;
+        ap.threads = std::min(most, std::max(32, work & ~31));
+        ap.smem = ((size_t)ap.plan.np * 16) << lg;
+    };
+    columns(c->py, c->nz, 1, false, o.tile_shift[1]);
+    columns(c->pz, c->ny, 1, false, o.tile_shift[2]);
+    columns(c->pzprop, c->ny, 1, true, o.tile_shift[3]);
+    columns(c->pz2, c->ny, 2, true, o.tile_shift[3]);
+    columns(c->py2, 1, 1, true, o.tile_shift[3]);
+    auto rows = [&](AxisPlan& ap, int work) {  // work: the most items of a line in a stage
+        const int64_t nrows = (int64_t)c->ny * c->nz;
+        int lines = std::max(1, many / work);
+        while (lines > 1 && (nrows + lines * W - 1) / (lines * W) * batch < 2 * (int64_t)sms) lines >>= 1;
+        ap.lines = std::max(1, lines >> o.tile_shift[0]);
+        ap.threads = std::min(kGenThreads, std::max(32, (ap.lines * work + 31) & ~31));
+        ap.smem = (size_t)ap.lines * ap.plan.np * 16;
+    };
+    rows(c->px, c->px.plan.nbmax);
+    if (c->px2.plan.nst) {
+        const GPlan& q = c->px2.plan;
+        int work = q.st[0].m / 2 + 1;
+        for (int i = 1; i < q.nst; ++i) work = std::max(work, q.st[i].nb);
+        rows(c->px2, work);
+    }
+}
+
 pfc_status fail(pfc_ctx* c, pfc_status s, const std::string& msg) {
     if (c) c->err = msg;
     return s;
@@ -440,8 +492,9 @@ bool same_class(const pfc_ctx* a, const pfc_step_params& pa, const pfc_ctx* b, c
            pa.mu == pb.mu && pa.lx == pb.lx && pa.ly == pb.ly && pa.lz == pb.lz && (pa.namp != 0.0) == (pb.namp != 0.0);
 }
 
-// A context of the shape and schedules of `like` holding m fields (batch = m).
-cudaError_t make_class_context(const pfc_ctx* like, int m, pfc_ctx** out) {
+// A context of the shape and schedules of `like` holding m fields (batch = m), one of
+// `classes` that run at the same time.
+cudaError_t make_class_context(const pfc_ctx* like, int m, int classes, pfc_ctx** out) {
     pfc_desc d{like->nx, like->ny, like->nz, like->dtype};
     pfc_ctx* c = nullptr;
     if (pfc_create_with(&d, &like->opt, &c) != PFC_OK) return cudaErrorMemoryAllocation;
@@ -459,6 +512,7 @@ cudaError_t make_class_context(const pfc_ctx* like, int m, pfc_ctx** out) {
     }
     c->batch = m;
     c->mstride = (int64_t)c->n_cmpl;
+    plan_launches(c, c->opt, m, std::max(1, c->num_sms / classes));
     *out = c;
     return cudaSuccess;
 }
@@ -662,48 +716,7 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
             return PFC_ERR_UNSUPPORTED;
         }
     }
-    // Lines per CTA of the general passes.  Columns: 128-byte segments (8 elements of 16 bytes:
-    // 16 FP32 or 8 FP64 columns), halved down to the 32-byte sectors of L2 while the tile's
-    // shared memory would leave fewer than three CTAs per SM, or the pass fewer than two CTAs
-    // per SM; then tile_shift times.  Threads: one butterfly each in the stage with the most, up
-    // to 256 (FP64: 128, for more CTAs per SM, unless the pass has too few CTAs for that); the
-    // update passes with few CTAs take one mode each, the update being their longest part.
-    // Rows: as many as fill those threads.
-    const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
-    const int many = c->dtype == PFC_F64 ? 128 : 256;
-    auto columns = [&](AxisPlan& ap, int64_t planes, int fields, bool update, int shift) {
-        const size_t line = (size_t)ap.plan.np * 16 * fields;
-        int lg = 3;
-        auto ctas = [&] { return ((c->nxh + (W << lg) - 1) / (W << lg)) * planes; };
-        while (lg > 1 && ((line << lg) > 72 * 1024 || ctas() < 2 * (int64_t)c->num_sms)) --lg;
-        while (lg > 0 && (line << lg) > kMaxDynSmem) --lg;
-        lg = std::max(0, lg - shift);
-        ap.lg = lg;
-        const bool few = ctas() < 4 * (int64_t)c->num_sms;
-        const int work = ((few && update ? ap.plan.n : ap.plan.nbmax * fields) << lg) + 31;
-        ap.threads = std::min(few ? kGenThreads : many, std::max(32, work & ~31));
-        ap.smem = ((size_t)ap.plan.np * 16) << lg;
-    };
-    columns(c->py, c->nz, 1, false, o.tile_shift[1]);
-    columns(c->pz, c->ny, 1, false, o.tile_shift[2]);
-    columns(c->pzprop, c->ny, 1, true, o.tile_shift[3]);
-    columns(c->pz2, c->ny, 2, true, o.tile_shift[3]);
-    columns(c->py2, 1, 1, true, o.tile_shift[3]);
-    auto rows = [&](AxisPlan& ap, int work) {  // work: the most items of a line in a stage
-        const int64_t nrows = (int64_t)c->ny * c->nz;
-        int lines = std::max(1, many / work);
-        while (lines > 1 && (nrows + lines * W - 1) / (lines * W) < 2 * (int64_t)c->num_sms) lines >>= 1;
-        ap.lines = std::max(1, lines >> o.tile_shift[0]);
-        ap.threads = std::min(kGenThreads, std::max(32, (ap.lines * work + 31) & ~31));
-        ap.smem = (size_t)ap.lines * ap.plan.np * 16;
-    };
-    rows(c->px, c->px.plan.nbmax);
-    if (c->px2.plan.nst) {
-        const GPlan& q = c->px2.plan;
-        int work = q.st[0].m / 2 + 1;
-        for (int i = 1; i < q.nst; ++i) work = std::max(work, q.st[i].nb);
-        rows(c->px2, work);
-    }
+    plan_launches(c, o, 1, c->num_sms);
     c->n_peak_blocks = peak_chunks(c->nx, c->ny, c->nz);
     // bond order starts with room for 4096 atoms and 64 neighbours each; pfc_bond_order
     // grows both when a call needs more (pfc_bond_reserve does it up front)
@@ -1377,7 +1390,7 @@ pfc_status pfc_ensemble_create(int n, pfc_ctx* const* ctxs, void* const* kpsis, 
         if (ce) break;
         const int m = (int)k.members.size();
         const pfc_ctx* like = e->ctx[k.members[0]];
-        ce = make_class_context(like, m, &k.cc);
+        ce = make_class_context(like, m, (int)e->cls.size(), &k.cc);
         if (!ce) ce = cudaMalloc(&k.state, like->state_bytes * m);
         if (!ce) ce = cudaMalloc((void**)&k.margs, sizeof(MemberArgs) * m);
         if (!ce) ce = cudaMalloc((void**)&k.ctr, sizeof(unsigned long long) * m);

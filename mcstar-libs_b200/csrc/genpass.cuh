@@ -21,8 +21,12 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
 // (six of 128; a radix-10 butterfly holds 40 of them, and its FP64 arithmetic needs more
 // temporaries).  They are latency-bound: at 128 registers and radices up to 16 the passes of
 // 240 x 200 x 180 FP32 took 0.025 / 0.049 / 0.088 ms (y, x, z) against 0.021 / 0.044 / 0.060.
+// The column passes may take the whole register file with one CTA: 1024 threads (FP64 768) of the
+// same registers, for fields with few tiles.
 template <typename T> constexpr int kGenCtas = sizeof(T) == 8 ? 3 : 4;
 constexpr int kGenThreads = 256;
+template <typename T> constexpr int kColThreads = sizeof(T) == 8 ? 768 : 1024;
+
 // largest first radix of the stepper's paired x pass (two butterflies in registers)
 constexpr int kPairRadix = 5;
 

@@ -15,7 +15,7 @@ namespace {
 // for bit, the one of the stepper's z pass (k_zprop).
 // ---------------------------------------------------------------------------------
 template <typename T, int DIR>
-__global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
+__global__ void __launch_bounds__(kColThreads<T>, 1)
     k_cols(const cx<T>* in, cx<T>* out, int ni, int64_t es, int64_t os, const __grid_constant__ GPlan p,
            const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, double scale, int64_t ms) {
     extern __shared__ __align__(16) unsigned char smem_raw[];

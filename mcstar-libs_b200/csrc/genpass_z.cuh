@@ -114,7 +114,7 @@ __device__ __forceinline__ cx<T> zmode(int prop, A&&... args) {
 // on the final step), the k = 0 mode from its FP64 slot.  The N^ lines (and with CARRY false
 // the psi^ lines beside them) stay in shared memory, digit-reversed, between the transforms.
 template <typename T, bool CARRY>
-__global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
+__global__ void __launch_bounds__(kColThreads<T>, 1)
     k_zprop(cx<T>* A, const cx<T>* B, int nx, int ny, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
             const int* __restrict__ tab, int lg, ZArgsT<T> a, const double2* __restrict__ k0, int* flag, int64_t ms,
             cx<T>* anext) {
