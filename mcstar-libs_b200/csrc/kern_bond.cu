@@ -80,24 +80,49 @@ template <> struct MaxRecB<float> { float i0, i1, i2; float field; };
 template <> struct MaxRecB<double> { double i0, i1, i2; float field; };
 
 // ---- compaction helpers -------------------------------------------------------------
+// Exclusive scan of nb counts (and their total) by one CTA: tiles of 8 counts per thread, warp
+// scans, a running total (a strided serial scan per thread took 8.3 us for 24 k counts, 7.2 now).
 __global__ void __launch_bounds__(1024) k_scan_b(const int* __restrict__ counts, int nb, int* __restrict__ offsets) {
-    __shared__ int part[1024];
-    const int chunk = (nb + 1023) / 1024;
-    const int b = threadIdx.x * chunk;
-    const int e = min(nb, b + chunk);
-    int s = 0;
-    for (int i = b; i < e; ++i) s += counts[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int v = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
+    constexpr int E = 8;
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int run = 0;
+    for (int base = 0; base < nb; base += 1024 * E) {
+        const int b = base + threadIdx.x * E;
+        int v[E], s = 0;
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            v[i] = b + i < nb ? counts[b + i] : 0;
+            s += v[i];
+        }
+        int inc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        __syncthreads();  // (the last tile's reads of wsum)
+        if (lane == 31) wsum[warp] = inc;
         __syncthreads();
-        part[threadIdx.x] += v;
+        if (warp == 0) {
+            int w = wsum[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += t;
+            }
+            wsum[lane] = w;
+        }
         __syncthreads();
+        int pos = run + inc - s + (warp ? wsum[warp - 1] : 0);
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            if (b + i < nb) offsets[b + i] = pos;
+            pos += v[i];
+        }
+        run += wsum[31];
     }
-    int run = part[threadIdx.x] - s;
-    for (int i = b; i < e; ++i) { offsets[i] = run; run += counts[i]; }
-    if (threadIdx.x == 1023) offsets[nb] = part[1023];
+    if (threadIdx.x == 0) offsets[nb] = run;
 }
 
 __device__ __forceinline__ int block_rank(bool f, int* wsum) {
@@ -165,132 +190,208 @@ __device__ __forceinline__ double get_diff(double x1, double x2, double w) {
     return fabs(d2) < fabs(d3) ? d2 : d3;
 }
 
-// kFill false: count the neighbours of atom i; true: also write them to list (whose
-// length the counting pass found).
-template <bool kFill>
-__device__ __forceinline__ void try_pair(const double* __restrict__ pos, int i, int j, double xi, double yi,
-                                         double zi, double box, double rlim, int* list, int& cnt, int& maxj) {
-    if (j == i) return;
-    const double dx = get_diff(pos[3 * j], xi, box);
-    const double dy = get_diff(pos[3 * j + 1], yi, box);
-    const double dz = get_diff(pos[3 * j + 2], zi, box);
-    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-    if (r <= rlim) {
-        if (kFill) list[cnt] = j;
-        ++cnt;
-        maxj = max(maxj, j);
+// Whether r = sqrt(d2) <= rlim, the root taken only within 1e-12 of the limit
+struct Within {
+    double rlim, lo, hi;
+    explicit Within(double r) : rlim(r), lo(r * r * (1.0 - 1e-12)), hi(r * r * (1.0 + 1e-12)) {
+        if (!(r > 1e-100)) {  // (no square to compare with: always the root)
+            lo = -1.0;
+            hi = INFINITY;
+        }
     }
-}
+    __device__ __forceinline__ bool operator()(double d2) const {
+        return d2 <= lo || (d2 <= hi && sqrt(d2) <= rlim);
+    }
+};
 
-// One thread per atom; nc == 0 selects all pairs (positions outside the box or a box too
-// small for three cells per side).  Counting pass (kFill false): nbc, maxjs.  Filling
-// pass: the list of atom i at nbr + nb_off[i], sorted by index (the reference sums over
-// neighbours in index order, bond-order.cpp:289-349).
+// One warp per atom, its lanes over the atoms of the 27 cells around it (about 80 candidates in
+// a crystal; a thread per atom left most of the GPU waiting for one dependent load after the
+// other: 24 k atoms 63 and 70 us; now 20 and 25).  nc == 0 selects all pairs (positions outside the box or a
+// box too small for three cells per side).  Counting pass (kFill false): nbc, maxjs.
+// Filling pass: the list of atom i at nbr + nb_off[i], sorted by index (the reference sums
+// over neighbours in index order, bond-order.cpp:289-349): each neighbour goes to its rank
+// among the atom's neighbours; lists longer than kNbList are sorted in place by one lane.
+constexpr int kNbWarps = 8, kNbList = 96;
 template <bool kFill>
-__global__ void k_neighbours(const double* __restrict__ pos, const int* __restrict__ np, double box, double rlim,
-                             int nc, const int* __restrict__ cell_off, const int* __restrict__ cell_atoms,
-                             const int* __restrict__ nb_off, int* __restrict__ nbr, int* __restrict__ nbc,
-                             int* __restrict__ maxjs) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * kNbWarps)
+    k_neighbours(const double* __restrict__ pos, const int* __restrict__ np, double box, Within within, int nc,
+                 const int* __restrict__ cell_off, const int* __restrict__ cell_atoms,
+                 const int* __restrict__ nb_off, int* __restrict__ nbr, int* __restrict__ nbc,
+                 int* __restrict__ maxjs) {
+    __shared__ int cell_end[kNbWarps][32], cell_at[kNbWarps][32], found[kNbWarps][kNbList];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * kNbWarps + w;
     const int P = *np;
     if (i >= P) return;
     const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-    int* list = kFill ? nbr + nb_off[i] : nullptr;
+    const bool fits = !kFill || nbc[i] <= kNbList;
+    int* list = kFill ? (fits ? found[w] : nbr + nb_off[i]) : nullptr;
     int cnt = 0, maxj = -1;
+    auto visit = [&](int j, bool valid) {
+        bool in = false;
+        if (valid && j != i) {
+            const double dx = get_diff(pos[3 * j], xi, box);
+            const double dy = get_diff(pos[3 * j + 1], yi, box);
+            const double dz = get_diff(pos[3 * j + 2], zi, box);
+            in = within(dx * dx + dy * dy + dz * dz);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            if (kFill) list[cnt + __popc(m & ((1u << lane) - 1u))] = j;
+            maxj = max(maxj, j);
+        }
+        cnt += __popc(m);
+    };
     if (nc == 0) {
-        for (int j = 0; j < P; ++j) try_pair<kFill>(pos, i, j, xi, yi, zi, box, rlim, list, cnt, maxj);
+        for (int j = lane; j - lane < P; j += 32) visit(j, j < P);
     } else {
-        const int cx = cell_of(xi, box, nc), cy = cell_of(yi, box, nc), cz = cell_of(zi, box, nc);
-        for (int dz = -1; dz <= 1; ++dz)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int c = (((cz + dz + nc) % nc) * nc + (cy + dy + nc) % nc) * nc + (cx + dx + nc) % nc;
-                    for (int k = cell_off[c]; k < cell_off[c + 1]; ++k)
-                        try_pair<kFill>(pos, i, cell_atoms[k], xi, yi, zi, box, rlim, list, cnt, maxj);
-                }
+        // lane c < 27: cell c of the neighbourhood, its first atom and the running count
+        int len = 0, at = 0;
+        if (lane < 27) {
+            const int cx = cell_of(xi, box, nc) + lane % 3 - 1, cy = cell_of(yi, box, nc) + lane / 3 % 3 - 1,
+                      cz = cell_of(zi, box, nc) + lane / 9 - 1;
+            const int c = ((cz + nc) % nc * nc + (cy + nc) % nc) * nc + (cx + nc) % nc;
+            at = cell_off[c];
+            len = cell_off[c + 1] - at;
+        }
+        int end = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += t;
+        }
+        cell_end[w][lane] = end;
+        cell_at[w][lane] = at - (end - len);  // + candidate number = index into cell_atoms
+        const int total = __shfl_sync(0xffffffffu, end, 31);
+        __syncwarp();
+        for (int f = lane; f - lane < total; f += 32) {
+            int c = 0;  // the first cell whose end is beyond f
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (cell_end[w][c + o - 1] <= f) c += o;
+            const bool valid = f < total;
+            visit(valid ? cell_atoms[cell_at[w][c] + f] : 0, valid);
+        }
     }
     if (!kFill) {
-        nbc[i] = cnt;
-        maxjs[i] = maxj;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) maxj = max(maxj, __shfl_xor_sync(0xffffffffu, maxj, o));
+        if (lane == 0) {
+            nbc[i] = cnt;
+            maxjs[i] = maxj;
+        }
         return;
     }
-    for (int a = 1; a < cnt; ++a) {  // insertion sort into index order
-        const int v = list[a];
-        int b = a - 1;
-        while (b >= 0 && list[b] > v) { list[b + 1] = list[b]; --b; }
-        list[b + 1] = v;
+    __syncwarp();
+    if (fits) {
+        int* out = nbr + nb_off[i];
+        for (int a = lane; a < cnt; a += 32) {
+            const int v = list[a];
+            int rank = 0;
+            for (int b = 0; b < cnt; ++b) rank += list[b] < v;
+            out[rank] = v;
+        }
+    } else if (lane == 0) {
+        for (int a = 1; a < cnt; ++a) {
+            const int v = list[a];
+            int b = a - 1;
+            while (b >= 0 && list[b] > v) { list[b + 1] = list[b]; --b; }
+            list[b + 1] = v;
+        }
     }
 }
 
-// q_lm for one (atom, l): thread t handles atom t/3, l = 4, 6, 8
-template <int L>
-__device__ void qlm_atom(const double* __restrict__ pos, int i, const int* __restrict__ list, int cnt, double box,
-                         double2* __restrict__ out, int lidx) {
-    double2 acc[2 * L + 1];
+// q_lm of every atom, l = 4, 6, 8: nine lanes per atom (three atoms per warp), lane m = 0 .. 8 for
+// +m and -m of all three l, whose P_l^m come from one upward recurrence in l.  The geometry of a
+// neighbour is computed once, by one of the nine lanes, and passed round by shuffles; the
+// sums over neighbours keep the list's order.  (A thread per atom and l: 132 us for 24 k atoms,
+// the recurrences and the geometry three times over with FP64 divisions; now 46 us, half of the
+// FP64 pipe.)
+__global__ void __launch_bounds__(128) k_qlm(const double* __restrict__ pos, const int* __restrict__ np,
+                                             const int* __restrict__ nbr, const int* __restrict__ nb_off,
+                                             const int* __restrict__ nbc, double box, double2* __restrict__ q) {
+    const int lane = threadIdx.x & 31, g = min(lane / 9, 2), m = lane < 27 ? lane - 9 * g : 0;
+    const int P = *np;
+    const int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 3 + g;
+    const bool mine = i < P && lane < 27;
+    const int cnt = i < P ? nbc[i] : 0;
+    const int most = max(__shfl_sync(0xffffffffu, cnt, 0),
+                         max(__shfl_sync(0xffffffffu, cnt, 9), __shfl_sync(0xffffffffu, cnt, 18)));
+    if (most == 0) return;
+    const int* list = nbr + (i < P ? nb_off[i] : 0);
+    double xi = 0.0, yi = 0.0, zi = 0.0;
+    if (i < P) { xi = pos[3 * i]; yi = pos[3 * i + 1]; zi = pos[3 * i + 2]; }
+    // (l + m - 1) / (l - m) and (2 l - 1) / (l - m) of the recurrence
+    double ra[9], rb[9];
 #pragma unroll
-    for (int m = 0; m < 2 * L + 1; ++m) acc[m] = make_double2(0.0, 0.0);
-    const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-    for (int a = 0; a < cnt; ++a) {
-        const int j = list[a];
-        const double dx = get_diff(pos[3 * j], xi, box);
-        const double dy = get_diff(pos[3 * j + 1], yi, box);
-        const double dz = get_diff(pos[3 * j + 2], zi, box);
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double x = dz / r;
-        const double rho = sqrt(dx * dx + dy * dy);
-        double2 eip = rho > 0.0 ? make_double2(dx / rho, dy / rho) : make_double2(1.0, 0.0);
-        const double s = sqrt(fmax(0.0, 1.0 - x * x));
-        const bool north = fabs(1.0 - x) < 1e-3, south = fabs(1.0 + x) < 1e-3;
-        double pmm = 1.0, fct = 1.0;
-        double2 em = make_double2(1.0, 0.0);
+    for (int l = 1; l <= 8; ++l) {
+        const double inv = l > m ? 1.0 / (double)(l - m) : 0.0;
+        ra[l] = (double)(2 * l - 1) * inv;
+        rb[l] = (double)(l + m - 1) * inv;
+    }
+    const double n4 = c_nlm[0][m], n6 = c_nlm[1][m], n8 = c_nlm[2][m];
+    double2 p4 = make_double2(0.0, 0.0), p6 = p4, p8 = p4, s4 = p4, s6 = p4, s8 = p4;  // sums for +m, -m
+    for (int a0 = 0; a0 < most; a0 += 9) {
+        double x = 0.0, sn = 0.0, ex = 1.0, ey = 0.0;
+        if (mine && a0 + m < cnt) {
+            const int j = list[a0 + m];
+            const double dx = get_diff(pos[3 * j], xi, box);
+            const double dy = get_diff(pos[3 * j + 1], yi, box);
+            const double dz = get_diff(pos[3 * j + 2], zi, box);
+            x = dz / sqrt(dx * dx + dy * dy + dz * dz);
+            const double rho = sqrt(dx * dx + dy * dy);
+            if (rho > 0.0) { ex = dx / rho; ey = dy / rho; }
+            sn = sqrt(fmax(0.0, 1.0 - x * x));
+        }
+        for (int b = 0; b < 9 && a0 + b < most; ++b) {
+            const int src = 9 * g + b;
+            const double xb = __shfl_sync(0xffffffffu, x, src), sb = __shfl_sync(0xffffffffu, sn, src);
+            const double cb = __shfl_sync(0xffffffffu, ex, src), db = __shfl_sync(0xffffffffu, ey, src);
+            if (a0 + b >= cnt) continue;
+            double pmm = 1.0, fct = 1.0;
+            double2 em = make_double2(1.0, 0.0);
 #pragma unroll
-        for (int m = 0; m <= L; ++m) {
-            if (m > 0) {
-                pmm = -pmm * fct * s;
+            for (int k = 1; k <= 8; ++k) {
+                if (k <= m) {
+                    pmm = -pmm * fct * sb;
+                    em = make_double2(em.x * cb - em.y * db, em.x * db + em.y * cb);
+                }
                 fct += 2.0;
-                em = make_double2(em.x * eip.x - em.y * eip.y, em.x * eip.y + em.y * eip.x);
             }
-            double plm;
-            if (m == L) plm = pmm;
-            else {
-                double p0 = pmm, p1 = x * (2 * m + 1) * pmm;
-                for (int ll = m + 2; ll <= L; ++ll) {
-                    const double p2 = (x * (2 * ll - 1) * p1 - (ll + m - 1) * p0) / (ll - m);
-                    p0 = p1; p1 = p2;
-                }
-                plm = p1;
+            double p0 = 0.0, p1 = m == 0 ? 1.0 : 0.0, v4 = 0.0, v6 = 0.0, v8 = 0.0;
+#pragma unroll
+            for (int l = 1; l <= 8; ++l) {
+                const double p2 = l == m ? pmm : xb * ra[l] * p1 - rb[l] * p0;  // (0 while l < m)
+                p0 = p1;
+                p1 = p2;
+                if (l == 4) v4 = n4 * p2;
+                if (l == 6) v6 = n6 * p2;
+                if (l == 8) v8 = n8 * p2;
             }
-            const double v = c_nlm[lidx][m] * plm;
-            if (m == 0) {
-                acc[L].x += v;
-            } else {
-                if (!north) { acc[L + m].x += v * em.x; acc[L + m].y += v * em.y; }
-                if (!south) {
-                    const double sg = (m & 1) ? -1.0 : 1.0;  // Y_l^-m = (-1)^m conj(Y_l^m)
-                    acc[L - m].x += sg * v * em.x;
-                    acc[L - m].y -= sg * v * em.y;
-                }
+            const bool north = fabs(1.0 - xb) < 1e-3, south = fabs(1.0 + xb) < 1e-3;
+            if (m == 0 || !north) {
+                p4.x += v4 * em.x; p4.y += v4 * em.y;
+                p6.x += v6 * em.x; p6.y += v6 * em.y;
+                p8.x += v8 * em.x; p8.y += v8 * em.y;
+            }
+            if (!south) {  // Y_l^-m = (-1)^m conj(Y_l^m)
+                s4.x += v4 * em.x; s4.y += v4 * em.y;
+                s6.x += v6 * em.x; s6.y += v6 * em.y;
+                s8.x += v8 * em.x; s8.y += v8 * em.y;
             }
         }
     }
-    const double inv = 1.0 / (double)cnt;
-#pragma unroll
-    for (int m = 0; m < 2 * L + 1; ++m) out[m] = make_double2(acc[m].x * inv, acc[m].y * inv);
-}
-
-__global__ void k_qlm(const double* __restrict__ pos, const int* __restrict__ np, const int* __restrict__ nbr,
-                      const int* __restrict__ nb_off, const int* __restrict__ nbc, double box,
-                      double2* __restrict__ q) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / 3, which = t - 3 * (t / 3);
-    if (i >= *np) return;
-    const int cnt = nbc[i];
-    if (cnt == 0) return;
-    const int* list = nbr + nb_off[i];
+    if (!mine || cnt == 0) return;
+    const double inv = 1.0 / (double)cnt, sg = (m & 1) ? -inv : inv;
     double2* qi = q + (size_t)i * kNQ;
-    if (which == 0) qlm_atom<4>(pos, i, list, cnt, box, qi, 0);
-    else if (which == 1) qlm_atom<6>(pos, i, list, cnt, box, qi + 9, 1);
-    else qlm_atom<8>(pos, i, list, cnt, box, qi + 22, 2);
+    if (m <= 4) qi[4 + m] = make_double2(p4.x * inv, p4.y * inv);
+    if (m <= 6) qi[9 + 6 + m] = make_double2(p6.x * inv, p6.y * inv);
+    qi[22 + 8 + m] = make_double2(p8.x * inv, p8.y * inv);
+    if (m > 0) {
+        if (m <= 4) qi[4 - m] = make_double2(s4.x * sg, -s4.y * sg);
+        if (m <= 6) qi[9 + 6 - m] = make_double2(s6.x * sg, -s6.y * sg);
+        qi[22 + 8 - m] = make_double2(s8.x * sg, -s8.y * sg);
+    }
 }
 
 __device__ __forceinline__ double sumsq(const double2* a, int n) {
@@ -298,100 +399,145 @@ __device__ __forceinline__ double sumsq(const double2* a, int n) {
     for (int m = 0; m < n; ++m) s += a[m].x * a[m].x + a[m].y * a[m].y;
     return s;
 }
-__device__ double wl4(const double2* q) {
-    double re = 0.0;
-    for (int k = 0; k < kW4; ++k) {
-        const int m1 = c_w4m[k][0], m2 = c_w4m[k][1], m3 = -m1 - m2;
-        const double2 a = q[m1 + 4], b = q[m2 + 4], c = q[m3 + 4];
-        const double2 ab = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-        re += c_w4[k] * (ab.x * c.x - ab.y * c.y);
-    }
-    const double s = sumsq(q, 9);
-    return re / sqrt(s * s * s);
-}
-__device__ double wl6(const double2* q) {
-    double re = 0.0;
-    for (int k = 0; k < kW6; ++k) {
-        const int m1 = c_w6m[k][0], m2 = c_w6m[k][1], m3 = -m1 - m2;
-        const double2 a = q[m1 + 6], b = q[m2 + 6], c = q[m3 + 6];
-        const double2 ab = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-        re += c_w6[k] * (ab.x * c.x - ab.y * c.y);
-    }
-    const double s = sumsq(q, 13);
-    return re / sqrt(s * s * s);
-}
-
 constexpr double kPi = 3.14159265358979323846;
 
-// per-atom invariants; rows of PFC_BOND_NCOL doubles for atoms with neighbours
-__global__ void __launch_bounds__(kBlk) k_bond_rows(const double* __restrict__ pos, const int* __restrict__ np,
-                                                    const int* __restrict__ nbr, const int* __restrict__ nb_off,
-                                                    const int* __restrict__ nbc,
-                                                    const int* __restrict__ maxjs, const double2* __restrict__ q,
-                                                    const int* __restrict__ row_off, double* __restrict__ rows,
-                                                    int row_capacity, int count_only, int* __restrict__ row_cnt) {
-    __shared__ int wsum[kBlk / 32];
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// sum over the terms k of w3j_k Re(q_m1 q_m2 q_m3), a warp's lanes over the terms
+__device__ __forceinline__ double wigner_sum(const double2* q, int l, const double* w3j, const int2* ms, int terms,
+                                             int lane) {
+    double re = 0.0;
+    for (int k = lane; k < terms; k += 32) {
+        const int2 m = ms[k];
+        const double2 a = q[m.x + l], b = q[m.y + l], c = q[l - m.x - m.y];
+        const double2 ab = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+        re += w3j[k] * (ab.x * c.x - ab.y * c.y);
+    }
+    return warp_sum(re);
+}
+
+// rows: atoms with neighbours, counted per block of kBlk atoms
+__global__ void __launch_bounds__(kBlk) k_row_count(const int* __restrict__ np, const int* __restrict__ nbc,
+                                                    int* __restrict__ row_cnt) {
     const int i = blockIdx.x * kBlk + threadIdx.x;
+    const int c = __syncthreads_count(i < *np && nbc[i] > 0);
+    if (threadIdx.x == 0) row_cnt[blockIdx.x] = c;
+}
+
+// Per-atom invariants; rows of PFC_BOND_NCOL doubles for atoms with neighbours.  A warp per atom:
+// its lanes hold the 39 components of q_lm (so that a neighbour's are read as one block), the
+// terms of the Wigner sums, and for xi half a warp each takes every other neighbour.  (A
+// thread per atom, 24 k atoms with 14 neighbours: 112 us, every load its own sector; now 79 us, bound
+// by the instructions of the sums: reducing all of them together, or the list by 32 entries,
+// changed nothing.)
+constexpr int kRowWarps = 8;
+__global__ void __launch_bounds__(32 * kRowWarps)
+    k_bond_rows(const double* __restrict__ pos, const int* __restrict__ np, const int* __restrict__ nbr,
+                const int* __restrict__ nb_off, const int* __restrict__ nbc, const int* __restrict__ maxjs,
+                const double2* __restrict__ q, const int* __restrict__ row_off, double* __restrict__ rows,
+                int row_capacity) {
+    __shared__ double w4[kW4], w6[kW6];
+    __shared__ int2 m4[kW4], m6[kW6];
+    __shared__ double2 own[kRowWarps][kNQ], last[kRowWarps][9];
+    __shared__ double sq[kRowWarps][kNQ], sqb[kRowWarps][kNQ], out[kRowWarps][PFC_BOND_NCOL];
+    for (int k = threadIdx.x; k < kW6; k += blockDim.x) {
+        w6[k] = c_w6[k];
+        m6[k] = make_int2(c_w6m[k][0], c_w6m[k][1]);
+        if (k < kW4) {
+            w4[k] = c_w4[k];
+            m4[k] = make_int2(c_w4m[k][0], c_w4m[k][1]);
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int P = *np;
-    const bool has = i < P && nbc[i] > 0;
-    if (count_only) {
-        const int c = __syncthreads_count(has);
-        if (threadIdx.x == 0) row_cnt[blockIdx.x] = c;
-        return;
-    }
-    const int rank = block_rank(has, wsum);
-    if (!has) return;
-    const int row = row_off[blockIdx.x] + rank;
-    if (row >= row_capacity) return;
-    const int cnt = nbc[i];
-    const int* list = nbr + nb_off[i];
-    const double2* qi = q + (size_t)i * kNQ;
-    double out[PFC_BOND_NCOL];
-    out[0] = pos[3 * i]; out[1] = pos[3 * i + 1]; out[2] = pos[3 * i + 2];
-    out[3] = (double)nbc[i];
-    // q_l
-    out[5] = sqrt(4.0 * kPi / 9.0 * sumsq(qi, 9));
-    out[6] = sqrt(4.0 * kPi / 13.0 * sumsq(qi + 9, 13));
-    out[7] = sqrt(4.0 * kPi / 17.0 * sumsq(qi + 22, 17));
-    out[8] = wl4(qi);
-    out[13] = wl6(qi + 9);
-    // q-bar_l, self included (bond-order.cpp:221-250)
-    const double invn = 1.0 / (1.0 + (double)nbc[i]);
-    const int lofs[3] = {0, 9, 22}, lw[3] = {9, 13, 17};
-    for (int li = 0; li < 3; ++li) {
-        double ss = 0.0;
-        for (int m = 0; m < lw[li]; ++m) {
-            double2 s = qi[lofs[li] + m];
+    for (int i = blockIdx.x * kRowWarps + w; i < P; i += gridDim.x * kRowWarps) {
+        const int cnt = nbc[i];
+        if (cnt == 0) continue;
+        // the row: the rows of the blocks before, and of the atoms before in this one
+        const int blk = i / kBlk;
+        int row = row_off[blk];
+        for (int t = blk * kBlk; t < i; t += 32) {
+            const int j = t + lane;
+            row += __popc(__ballot_sync(0xffffffffu, j < i && nbc[j] > 0));
+        }
+        if (row >= row_capacity) continue;
+        const int* list = nbr + nb_off[i];
+        const double2* qi = q + (size_t)i * kNQ;
+        const double invn = 1.0 / (1.0 + (double)cnt);
+        for (int c = lane; c < kNQ; c += 32) {
+            const double2 v = qi[c];
+            own[w][c] = v;
+            sq[w][c] = v.x * v.x + v.y * v.y;
+            double2 s = v;  // q-bar_l, self included (bond-order.cpp:221-250)
             for (int a = 0; a < cnt; ++a) {
-                const double2 o = q[(size_t)list[a] * kNQ + lofs[li] + m];
-                s.x += o.x; s.y += o.y;
+                const double2 o = q[(size_t)list[a] * kNQ + c];
+                s.x += o.x;
+                s.y += o.y;
             }
-            s.x *= invn; s.y *= invn;
-            ss += s.x * s.x + s.y * s.y;
+            s.x *= invn;
+            s.y *= invn;
+            sqb[w][c] = s.x * s.x + s.y * s.y;
         }
-        out[9 + li] = sqrt(4.0 * kPi / (double)lw[li] * ss);
-    }
-    // w4b as the reference computes it: the last neighbour's q4m divided by Nb
-    {
-        double2 qb[9];
-        const double2* ql = q + (size_t)maxjs[i] * kNQ;
-        for (int m = 0; m < 9; ++m) qb[m] = make_double2(ql[m].x / (double)nbc[i], ql[m].y / (double)nbc[i]);
-        out[12] = wl4(qb);
-    }
-    // xi: neighbours with normalised q6 . conj(q6) > 0.7 (bond-order.cpp:267-287)
-    {
-        const double2* q6 = qi + 9;
-        const double ni = sqrt(sumsq(q6, 13));
-        int s = 0;
-        for (int a = 0; a < cnt; ++a) {
-            const double2* o = q + (size_t)list[a] * kNQ + 9;
-            double d = 0.0;
-            for (int m = 0; m < 13; ++m) d += q6[m].x * o[m].x + q6[m].y * o[m].y;
-            if (d / (ni * sqrt(sumsq(o, 13))) > 0.7) ++s;
+        if (lane < 9) {  // w4b as the reference computes it: the last neighbour's q4m divided by Nb
+            const double2 v = q[(size_t)maxjs[i] * kNQ + lane];
+            last[w][lane] = make_double2(v.x / (double)cnt, v.y / (double)cnt);
         }
-        out[4] = (double)s;
+        __syncwarp();
+        const double r4 = wigner_sum(own[w], 4, w4, m4, kW4, lane), r6 = wigner_sum(own[w] + 9, 6, w6, m6, kW6, lane),
+                     rb = wigner_sum(last[w], 4, w4, m4, kW4, lane);
+        // xi: neighbours with normalised q6 . conj(q6) > 0.7 (bond-order.cpp:267-287)
+        double n6 = 0.0;
+        for (int m = 0; m < 13; ++m) n6 += sq[w][9 + m];
+        const double ni = sqrt(n6);
+        const int hl = lane & 15, half = lane >> 4;
+        const double2 mine = hl < 13 ? own[w][9 + hl] : make_double2(0.0, 0.0);
+        int solid = 0;
+        for (int a = half; a - half < cnt; a += 2) {
+            double d = 0.0, s = 0.0;
+            if (a < cnt && hl < 13) {
+                const double2 o = q[(size_t)list[a] * kNQ + 9 + hl];
+                d = mine.x * o.x + mine.y * o.y;
+                s = o.x * o.x + o.y * o.y;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                d += __shfl_xor_sync(0xffffffffu, d, o);
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+            }
+            // d / (sqrt(n6) sqrt(s)) > 0.7, the roots taken only within 1e-12 of it
+            const double d2 = d * d, lim = 0.49 * (n6 * s);
+            if (a < cnt && d > 0.0 && (d2 > lim * (1.0 + 1e-12) || (!(d2 < lim * (1.0 - 1e-12)) && d / (ni * sqrt(s)) > 0.7)))
+                ++solid;
+        }
+        solid += __shfl_xor_sync(0xffffffffu, solid, 16);
+        if (lane < 3) {
+            out[w][lane] = pos[3 * i + lane];
+            const int o = lane == 0 ? 0 : lane == 1 ? 9 : 22, n = lane == 0 ? 9 : lane == 1 ? 13 : 17;
+            double s = 0.0, sb = 0.0;
+            for (int m = 0; m < n; ++m) {
+                s += sq[w][o + m];
+                sb += sqb[w][o + m];
+            }
+            out[w][5 + lane] = sqrt(4.0 * kPi / (double)n * s);
+            out[w][9 + lane] = sqrt(4.0 * kPi / (double)n * sb);
+            if (lane == 0) {
+                out[w][3] = (double)cnt;
+                out[w][4] = (double)solid;
+                out[w][8] = r4 / sqrt(s * s * s);
+                const double l2 = sumsq(last[w], 9);
+                out[w][12] = rb / sqrt(l2 * l2 * l2);
+            }
+            if (lane == 1) out[w][13] = r6 / sqrt(s * s * s);
+        }
+        __syncwarp();
+        if (lane < PFC_BOND_NCOL) rows[(size_t)row * PFC_BOND_NCOL + lane] = out[w][lane];
+        __syncwarp();  // before the next atom's values
     }
-    for (int c = 0; c < PFC_BOND_NCOL; ++c) rows[(size_t)row * PFC_BOND_NCOL + c] = out[c];
 }
 
 double fact(int n) { double r = 1.0; for (int k = 2; k <= n; ++k) r *= k; return r; }
@@ -473,8 +619,11 @@ cudaError_t bond_reserve(pfc_ctx* c, int atoms, int64_t pairs) {
 
 cudaError_t launch_bond_order(pfc_ctx* c, const void* maxima, int n, double h0, double h1, double h2, double ths,
                               double boxsize, double rlim, double* out_rows, int row_capacity, int* n_rows_host) {
-    cudaError_t e = upload_tables();
-    if (e) return e;
+    cudaError_t e = cudaSuccess;
+    if (!c->bond_tables) {
+        if ((e = upload_tables())) return e;
+        c->bond_tables = true;
+    }
     if ((e = bond_reserve(c, n, 0))) return e;
     BondScratch s;
     scratch_layout(c->max_atoms, &s, (char*)c->bond_scratch);
@@ -514,23 +663,25 @@ cudaError_t launch_bond_order(pfc_ctx* c, const void* maxima, int n, double h0, 
         k_cell_fill<<<pb, 256, 0, st>>>(s.pos, np, boxsize, nc, s.cell_off, s.cell_fill, s.cell_atoms);
     }
     // 3. neighbour lists: count, scan into list offsets, grow the pair buffer, fill
-    k_neighbours<false><<<pb, 256, 0, st>>>(s.pos, np, boxsize, rlim, nc, s.cell_off, s.cell_atoms, nullptr, nullptr,
-                                            s.nb, s.maxj);
+    const int nwb = (P + kNbWarps - 1) / kNbWarps;
+    const Within within(rlim);
+    k_neighbours<false><<<nwb, 32 * kNbWarps, 0, st>>>(s.pos, np, boxsize, within, nc, s.cell_off, s.cell_atoms,
+                                                       nullptr, nullptr, s.nb, s.maxj);
     k_scan_b<<<1, 1024, 0, st>>>(s.nb, P, s.nb_off);
     if ((e = cudaGetLastError())) return e;
     int pairs = 0;
     if ((e = cudaMemcpyAsync(&pairs, s.nb_off + P, sizeof(int), cudaMemcpyDeviceToHost, st))) return e;
     if ((e = cudaStreamSynchronize(st))) return e;
     if ((e = bond_reserve(c, 0, pairs))) return e;
-    k_neighbours<true><<<pb, 256, 0, st>>>(s.pos, np, boxsize, rlim, nc, s.cell_off, s.cell_atoms, s.nb_off,
-                                           c->bond_pairs, nullptr, nullptr);
-    k_qlm<<<(3 * P + 127) / 128, 128, 0, st>>>(s.pos, np, c->bond_pairs, s.nb_off, s.nb, boxsize, s.q);
+    k_neighbours<true><<<nwb, 32 * kNbWarps, 0, st>>>(s.pos, np, boxsize, within, nc, s.cell_off, s.cell_atoms,
+                                                      s.nb_off, c->bond_pairs, s.nb, nullptr);
+    k_qlm<<<(P + 11) / 12, 128, 0, st>>>(s.pos, np, c->bond_pairs, s.nb_off, s.nb, boxsize, s.q);
     const int rb = (P + kBlk - 1) / kBlk;
-    k_bond_rows<<<rb, kBlk, 0, st>>>(s.pos, np, c->bond_pairs, s.nb_off, s.nb, s.maxj, s.q, nullptr, nullptr, 0, 1,
-                                     s.row_cnt);
+    k_row_count<<<rb, kBlk, 0, st>>>(np, s.nb, s.row_cnt);
     k_scan_b<<<1, 1024, 0, st>>>(s.row_cnt, rb, s.row_off);
-    k_bond_rows<<<rb, kBlk, 0, st>>>(s.pos, np, c->bond_pairs, s.nb_off, s.nb, s.maxj, s.q, s.row_off, out_rows,
-                                     row_capacity, 0, s.row_cnt);
+    // (the Wigner tables are copied into shared memory once per CTA: a grid that fills the GPU)
+    k_bond_rows<<<std::min((P + kRowWarps - 1) / kRowWarps, 4 * c->num_sms), 32 * kRowWarps, 0, st>>>(
+        s.pos, np, c->bond_pairs, s.nb_off, s.nb, s.maxj, s.q, s.row_off, out_rows, row_capacity);
     if ((e = cudaGetLastError())) return e;
     int rows = 0;
     if ((e = cudaMemcpyAsync(&rows, s.row_off + rb, sizeof(int), cudaMemcpyDeviceToHost, st))) return e;

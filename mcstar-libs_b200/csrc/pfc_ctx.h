@@ -61,6 +61,7 @@ struct pfc_ctx {
     size_t bond_scratch_bytes;
     int64_t max_pairs;
     int* bond_pairs;
+    bool bond_tables = false;     // the constant tables are on this context's device
     int fused_z;                  // 0: general z pass; otherwise the register z kernel variant id
     int z_carry;                  // carry psi^ itself instead of A: standard layout, A = IFFT_z(psi^)/nz
                                   // in work2; tiled, psi^ z-tiled in work2 and A in the psi^ buffer

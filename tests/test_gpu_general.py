@@ -98,3 +98,24 @@ def test_paired_x_pass(shape, dtype):
     st.step(3)
     want = O.step(k0, 3, 0.25, 0.3, st.lens, shape)
     assert rel(st.kspace(), want) < (2e-6 if dtype == F32 else 1e-12)
+
+
+@pytest.mark.parametrize("n,box,rlim", [(1, 50.0, 5.0), (2, 50.0, 40.0), (33, 30.0, 8.0), (150, 12.0, 12.0),
+                                        (700, 40.0, 12.5), (900, 64.0, 9.0)])
+def test_bond_order_lists(n, box, rlim):
+    """Bond order at the neighbour lists' edges: no neighbours, all pairs (fewer than three cells per
+    side), lists beyond the 96 entries a warp sorts in shared memory, several blocks of rows."""
+    from mcstar_b200 import Context, maximum_dtype
+    import torch
+    rng = np.random.default_rng(n)
+    idx = rng.uniform(0, box, (n, 3)).astype(F32)
+    field = rng.uniform(-0.1, 1.0, n).astype(F32)
+    M = np.zeros(n, dtype=maximum_dtype(F32))
+    M["i0"], M["i1"], M["i2"], M["field"] = idx[:, 0], idx[:, 1], idx[:, 2], field
+    ctx = Context((8, 8, 8), F32)
+    dev = torch.from_numpy(M.view(np.uint8).ravel().copy()).cuda()
+    rows = ctx.bond_order(dev, n, (1.0, 1.0, 1.0), 0.0, box, rlim).cpu().numpy()
+    res, _ = O.bond_order(idx, field, (1.0, 1.0, 1.0), 0.0, box, rlim)
+    assert rows.shape[0] == len(res["x"])
+    for i, c in enumerate(O.BOND_COLUMNS):
+        np.testing.assert_allclose(rows[:, i], res[c], atol=1e-9, rtol=1e-9, err_msg=c)
