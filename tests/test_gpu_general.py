@@ -119,3 +119,22 @@ def test_bond_order_lists(n, box, rlim):
     assert rows.shape[0] == len(res["x"])
     for i, c in enumerate(O.BOND_COLUMNS):
         np.testing.assert_allclose(rows[:, i], res[c], atol=1e-9, rtol=1e-9, err_msg=c)
+
+
+def test_status_words_between_calls():
+    """The stepper clears its status words only after a call that found one set: a bad state is
+    reported by the call that meets it and by no later one, however good and bad calls alternate."""
+    from mcstar_b200 import PfcError
+    from test_gpu_step import stepper
+    shape = (48, 40, 1)
+    psi = -0.2 + 0.05 * np.random.default_rng(2).uniform(-1, 1, shape[::-1])
+    st = stepper(shape, F32)
+    for bad in (False, False, True, True, False, True, False, False):
+        st.set_real(psi)
+        if bad:
+            st.kpsi[10] = float("nan")
+            with pytest.raises(PfcError):
+                st.step(1)
+        else:
+            st.step(1)
+            assert np.isfinite(st.real()).all()
