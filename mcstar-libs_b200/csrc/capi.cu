@@ -226,25 +226,21 @@ void free_ctx(pfc_ctx* c) {
                     c->peak_mask};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    if (c->host) cudaFreeHost(c->host);
     delete c;
 }
 
-// Copies a small result (up to kHostBytes) to dst and waits for the context's stream: through
-// the context's pinned memory, which the copy engine writes itself (a copy to pageable memory
-// is staged by the driver), or straight where that could not be had. With the status words
-// cleared only where needed, one FP32 step of a 128^2 film: 40.5 -> 37.2 us per call.
-constexpr size_t kHostBytes = 256;
+// Copies a small result to dst and waits for the context's stream. (Through pinned memory of
+// the context the step of a 128^2 film took 37.2 instead of 38.4 us, but its allocation 1.4 to
+// 4 ms of pfc_create's 1.5.)
 cudaError_t read_back(pfc_ctx* c, void* dst, const void* src, size_t bytes) {
-    void* to = c->host ? c->host : dst;
-    cudaError_t e = cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, c->stream);
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream);
     if (!e) e = cudaStreamSynchronize(c->stream);
-    if (!e && c->host) std::memcpy(dst, c->host, bytes);
     return e;
 }
 
 // The stepper's status words, cleared unless they are known to be clear (they stay so until a
-// call reads a set one, fails, or is one that does not clear them).
+// call reads a set one, fails, or is one that does not clear them): a memset before the launches
+// of a single step of a 128^2 film is 1.6 of 40 us.
 cudaError_t clear_flag(pfc_ctx* c) {
     const bool clear = c->flag_clear;
     c->flag_clear = false;
@@ -697,8 +693,8 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     // (two z transforms; 0.344 against 0.447 ms at 512^3) and no FP32 round trip of the state
     // through IFFT_z / FFT_z each step (its FP32 error against FP64 is the reference cuFFT
     // path's or lower at 1, 10, 100, 1000 steps); elsewhere A.
-    // The general (Stockham) z pass carries psi^ too unless the options ask for A: one
-    // transform fewer per column, the kernels being issue-bound at the lengths they serve.
+    // The general z pass carries psi^ too unless the options ask for A: one transform fewer
+    // per column, and no FP32 round trip of the state.
     const bool gen_carry = !c->fused_z && c->nz > 1 && o.z_carry != 0;
     const bool carry =
         gen_carry || (c->fused_z && (o.z_carry == 1 || (o.z_carry == -1 && c->tiled && c->fused_z == 6)));
@@ -791,10 +787,6 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     }
     if (e == cudaSuccess) e = cudaMemcpy(c->fft_tab, itab.data(), itab.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(c->flag, 0, sizeof(int) * 4);
-    if (e == cudaSuccess && cudaMallocHost(&c->host, kHostBytes) != cudaSuccess) {
-        cudaGetLastError();
-        c->host = nullptr;
-    }
     if (e == cudaSuccess) e = set_fft_attributes(c);
     if (e == cudaSuccess && c->fused_z) e = set_zcol_attributes(c);
     if (e == cudaSuccess && c->fused_y) e = set_pass_attributes(c);

@@ -51,7 +51,6 @@ struct pfc_ctx {
     double2* k0;                  // FP64 k = 0 mode carried by the stepper
     int* flag;                    // device status word of the stepper (non-finite watchdog)
     bool flag_clear = false;      // every word of flag is known to be zero
-    void* host = nullptr;         // pinned host memory for small results (null: none was to be had)
     uint32_t* peak_mask;          // one bit per cell (peak finder)
     int* peak_counts;             // set bits per chunk of the mask
     int* peak_offsets;            // exclusive scan of peak_counts (+ total)
