@@ -43,12 +43,12 @@ template <typename T> struct ZColumn {
         : kx(kx_), kk0(kwave_ck<T>(kx_, nx, a.ckx)), kxy(kk0 * kk0 + k1 * k1) {}
 };
 
-// 1 / d, d >= 1: in FP32 the approximate reciprocal and one Newton step (within an ulp) in
-// place of the division's dozen instructions.
+// 1 / d: in FP32 the approximate reciprocal and one Newton step (within an ulp) in place of the
+// division's dozen instructions. Where the step has no number (d zero, infinite or NaN: a D that
+// overflowed, or bad parameters) the approximation stands, which is the division's value.
 __device__ __forceinline__ float recip(float d) {
-    d = fminf(d, 1e38f);  // (an overflowed D gives 0, as the division did)
-    const float r = __fdividef(1.0f, d);
-    return fmaf(r, fmaf(-d, r, 1.0f), r);
+    const float r = __fdividef(1.0f, d), e = fmaf(-d, r, 1.0f);
+    return e == e ? fmaf(r, e, r) : r;
 }
 __device__ __forceinline__ double recip(double d) { return 1.0 / d; }
 

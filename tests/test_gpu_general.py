@@ -138,3 +138,15 @@ def test_status_words_between_calls():
         else:
             st.step(1)
             assert np.isfinite(st.real()).all()
+
+
+@pytest.mark.parametrize("dtype", [F32, F64], ids=["f32", "f64"])
+@pytest.mark.parametrize("shape", [(24, 20, 1), (20, 18, 12)], ids=str)
+def test_nonfinite_parameters_are_reported(shape, dtype):
+    """A NaN in the propagator reaches the new state, and the call reports it."""
+    from mcstar_b200 import PfcError
+    from test_gpu_step import stepper
+    st = stepper(shape, dtype, eps=float("nan"))
+    st.set_real(-0.2 + 0.05 * np.random.default_rng(2).uniform(-1, 1, shape[::-1]))
+    with pytest.raises(PfcError):
+        st.step(2)
