@@ -50,7 +50,7 @@ def _sync():
 
 class CufftPlan:
     """``CufftPlan<F, R2C|C2R>(int3 shape)``; ``execute(in, out)`` runs the unnormalised
-    transform with this library's Stockham FFT (no cuFFT)."""
+    transform with this library's own FFT (no cuFFT)."""
 
     def __init__(self, dtype, kind, shape):
         self.dtype = np.dtype(dtype)
