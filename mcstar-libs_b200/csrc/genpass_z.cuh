@@ -116,7 +116,7 @@ __device__ __forceinline__ cx<T> zmode(int prop, A&&... args) {
 template <typename T, bool CARRY>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_zprop(cx<T>* A, const cx<T>* B, int nx, int ny, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
-            const int* __restrict__ tab, int lg, ZArgsT<T> a, const double2* __restrict__ k0, int* flag, int64_t ms,
+            const int* __restrict__ tab, int lg, ZArgsT<T> a, const double2* k0, int* flag, int64_t ms,
             cx<T>* anext) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);

@@ -328,7 +328,7 @@ __device__ __forceinline__ void row_tiles_r2c(const float2* rb, const float2* tw
 // cufft_wrapper.hpp:61-86.
 template <class X, int MODE>
 __global__ void __launch_bounds__(X::T, X::MINB)
-    k_xrow(const float2* in, float2* out, const float* __restrict__ pot, int nrows, const float2* __restrict__ twg,
+    k_xrow(const float2* in, float2* out, const float* pot, int nrows, const float2* __restrict__ twg,
            float mul, float Cc, float mu, int64_t ms) {
     constexpr int NX = X::NX, M = X::M, NXH = X::NXH, E = X::E, P = X::P, U = X::U, R = X::R, LDR = X::LDR;
     in += blockIdx.z * ms;  // fields of a batch (grid z; no potential then)

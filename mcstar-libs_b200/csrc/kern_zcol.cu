@@ -225,11 +225,10 @@ __device__ __forceinline__ void store_state(float2 (&v)[Z::E], float2* A, int64_
     }
 }
 
-// lay bits 0, 1, 2: A, B, O kx-tiled (col_addr); O may be A when their layouts agree.
+// lay bits 0, 1, 2: A, B, O kx-tiled (col_addr); O may be A or B when their layouts agree.
 template <class Z, int PROP>
-__global__ void __launch_bounds__(Z::T, Z::MINB) k_zcol(const float2* A, const float2* __restrict__ B, float2* O,
-                                                   int nx, int ny, int lay, ZArgsF a,
-                                                   const double2* __restrict__ k0, int* flag,
+__global__ void __launch_bounds__(Z::T, Z::MINB) k_zcol(const float2* A, const float2* B, float2* O,
+                                                   int nx, int ny, int lay, ZArgsF a, const double2* k0, int* flag,
                                                    const float2* __restrict__ twg, int64_t ms) {
     constexpr int NZ = Z::NZ, E = Z::E, TX = Z::TX, P = Z::P, U = Z::U, TH = Z::TH;
     A += blockIdx.z * ms;  // fields of a batch (grid z)
@@ -410,7 +409,7 @@ __device__ __forceinline__ void propagate3(float2 (&v)[Z::E], float2* tile, int 
 
 // LAY: the layouts of A, B, O as k_zcol's lay, fixed at compile time (0, 1 or 7)
 template <class Z, int LAY, int PROP>
-__global__ void __launch_bounds__(Z::T, 2) k_zcol3(const float2* A, const float2* __restrict__ B, float2* O, int nx,
+__global__ void __launch_bounds__(Z::T, 2) k_zcol3(const float2* A, const float2* B, float2* O, int nx,
                                                     int ny, ZArgsF a, const double2* __restrict__ k0, int* flag,
                                                     const float2* __restrict__ twg, int64_t ms) {
     constexpr int NZ = Z::NZ, E = Z::E, TX = Z::TX, P = Z::P, TH = Z::TH;
@@ -484,8 +483,8 @@ __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_grou
 // round trip of the state per step (its rounding matches the reference's k-space
 // update), and one more read and write of the state.
 template <class Z, int PROP>
-__global__ void __launch_bounds__(Z::TH, Z::CMINB) k_zcarry(float2* kpsi, float2* A, const float2* __restrict__ B, int nx,
-                                                      int ny, ZArgsF a, const double2* __restrict__ k0, int* flag,
+__global__ void __launch_bounds__(Z::TH, Z::CMINB) k_zcarry(float2* kpsi, float2* A, const float2* B, int nx,
+                                                      int ny, ZArgsF a, const double2* k0, int* flag,
                                                       const float2* __restrict__ twg, int64_t ms) {
     constexpr int NZ = Z::NZ, E = Z::E, TX = Z::TX, P = Z::P, TH = Z::TH;
     static_assert(TX == 8 && (Z::U == 1 || Z::U == 2), "staging swizzle assumes 8 columns per tile");
