@@ -8,188 +8,12 @@
 #include <vector>
 #include "bulk.cuh"
 #include "chain.cuh"
-#include "genpass.cuh"
+#include "genplan.h"
 #include "pfc_ctx.h"
 
 using namespace pfc;
 
 namespace {
-
-// The stages of an n-point plan of the general engine (genfft.cuh), in order.  order 0: the
-// fewest stages with radices up to `cap`, as equal as possible (the least sum), larger
-// radices first; 1: radices up to 5 (4 before 2); 2: as 0 with the odd radices first.  Primes
-// from 7 to kMaxOddRadix are stages of their own.  At least two stages, the last with a
-// hand-written DFT: a stage of radix 1 is appended where needed.  first > 0: only plans without
-// primes whose smallest radix is at most that, in ascending order.
-bool factor_radices(int n, std::vector<int>& rs, int order, int cap, int first) {
-    rs.clear();
-    if (n < 1) return false;
-    std::vector<int> primes;
-    for (int p = 7; p <= kMaxOddRadix; p += 2) {
-        bool prime = true;
-        for (int d = 3; d * d <= p; d += 2) prime = prime && (p % d != 0);
-        if (!prime) continue;
-        while (n % p == 0) { primes.push_back(p); n /= p; }
-    }
-    std::vector<int> best;
-    if (first > 0 && !primes.empty()) return false;
-    if (order == 1) {
-        for (int r : {4, 2, 3, 5})
-            while (n % r == 0) { best.push_back(r); n /= r; }
-        if (n != 1) return false;
-    } else {
-        static const int kRadix[] = {10, 9, 8, 6, 5, 4, 3, 2};
-        std::vector<int> cur;
-        int best_len = kMaxStages + 1, best_sum = 0;
-        // descending factorisations of n; the number of stages bounded by the best so far
-        auto search = [&](auto&& self, int rest, int from) -> void {
-            if (rest == 1) {
-                if (first > 0 && (cur.empty() || cur.back() > first)) return;
-                const int len = (int)cur.size();
-                int sum = 0;
-                for (int r : cur) sum += r;
-                if (len < best_len || (len == best_len && sum < best_sum)) {
-                    best = cur;
-                    best_len = len;
-                    best_sum = sum;
-                }
-                return;
-            }
-            if ((int)cur.size() >= best_len) return;
-            for (int i = from; i < (int)(sizeof(kRadix) / sizeof(kRadix[0])); ++i)
-                if (rest % kRadix[i] == 0 && kRadix[i] <= cap) {
-                    cur.push_back(kRadix[i]);
-                    self(self, rest / kRadix[i], i);
-                    cur.pop_back();
-                }
-        };
-        search(search, n, 0);
-        if (best_len > kMaxStages) return false;
-        if (order == 2) std::stable_partition(best.begin(), best.end(), [](int r) { return r % 2 != 0; });
-    }
-    if (first > 0) {
-        std::sort(best.begin(), best.end());
-        if (best.empty() || best[0] > first) return false;
-    }
-    rs = primes;
-    rs.insert(rs.end(), best.begin(), best.end());
-    if (best.empty() || rs.size() < 2) rs.push_back(1);
-    if (rs.size() < 2) rs.push_back(1);
-    return (int)rs.size() <= kMaxStages;
-}
-
-// Makes an n-point plan: appends its twiddles to tab (forward sign, FP64) and its index
-// tables to itab.
-bool make_plan(int n, GPlan& p, std::vector<std::complex<double>>& tab, std::vector<int>& itab, int order, int cap,
-               int first = 0) {
-    std::vector<int> rs;
-    if (!factor_radices(n, rs, order, cap, first)) return false;
-    std::memset(&p, 0, sizeof(p));
-    p.n = n;
-    p.nst = (int)rs.size();
-    p.rl = rs.back();
-    p.pad = p.rl % 2 == 0;
-    p.kstep = n / p.rl;
-    p.np = n + p.pad * p.kstep;
-    p.by_rl = make_fastdiv(p.rl);
-    p.by_n = make_fastdiv(n);
-    auto padded = [&](int i) { return i + p.pad * (i / p.rl); };
-    int M = n;
-    for (int s = 0; s < p.nst; ++s) {
-        GStage& g = p.st[s];
-        g.R = rs[s];
-        g.m = M / g.R;
-        g.nb = n / g.R;
-        p.nbmax = std::max(p.nbmax, g.nb);
-        g.ms = s == p.nst - 1 ? 1 : padded(g.m);
-        g.Ms = padded(M);
-        g.by_m = make_fastdiv(g.m);
-        g.by_nb = make_fastdiv(g.nb);
-        g.tw = (int)tab.size();
-        for (int r = 1; r < g.R; ++r)
-            for (int j = 0; j < g.m; ++j) {
-                const double ang = -2.0 * M_PI * (double)(((long long)r * j) % M) / (double)M;
-                tab.emplace_back(std::cos(ang), std::sin(ang));
-            }
-        g.rt = (int)tab.size();
-        if (g.R >= 7 && g.R % 2 && g.R != 9)
-            for (int q = 0; q < g.R; ++q) {
-                const double ang = -2.0 * M_PI * (double)q / (double)g.R;
-                tab.emplace_back(std::cos(ang), std::sin(ang));
-            }
-        M = g.m;
-    }
-    // frequency of position q: digits of q by the stages, reversed
-    std::vector<int> freq(n);
-    for (int q = 0; q < n; ++q) {
-        int rest = q, k = 0, w = 1;
-        for (int s = 0; s < p.nst; ++s) {
-            const int d = rest / p.st[s].m;
-            rest -= d * p.st[s].m;
-            k += d * w;
-            w *= p.st[s].R;
-        }
-        freq[q] = k;
-    }
-    p.rev = (int)itab.size();
-    for (int b = 0; b < p.kstep; ++b) itab.push_back(freq[b * p.rl]);
-    p.pos = (int)itab.size();
-    itab.resize(itab.size() + n);
-    for (int q = 0; q < n; ++q) itab[p.pos + freq[q]] = padded(q);
-    return true;
-}
-
-// Lines per CTA and threads of the general passes for `batch` fields on `sms` multiprocessors (a
-// class of an ensemble shares the GPU with the other classes).
-void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) {
-    // Columns: 128-byte segments (8 elements of 16 bytes:
-    // 16 FP32 or 8 FP64 columns), halved down to the 32-byte sectors of L2 while the tile's
-    // shared memory would leave fewer than three CTAs per SM, or the pass fewer than two CTAs
-    // per SM; then tile_shift times.  Threads: one butterfly each in the stage with the most, up
-    // to 256 (FP64: 128, for more CTAs per SM); a pass with at most four CTAs per SM takes 256, with
-    // at most two the SM's whole register file, and an update pass with few CTAs one mode per
-    // thread: the update is its longest part (1000^2 FP32 step, 126 CTAs: 46.3 us at 256 threads,
-    // 28.3 at 1000; with noise 59.6 and 31.7; two-column tiles at 256 threads 33.4 and 34.0).
-    // Rows: as many as fill those threads.
-    const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
-    const int many = c->dtype == PFC_F64 ? 128 : 256;
-    auto columns = [&](AxisPlan& ap, int64_t planes, int fields, bool update, int shift) {
-        const size_t line = (size_t)ap.plan.np * 16 * fields;
-        int lg = 3;
-        auto ctas = [&] { return ((c->nxh + (W << lg) - 1) / (W << lg)) * planes * batch; };
-        while (lg > 1 && ((line << lg) > 72 * 1024 || ctas() < 2 * (int64_t)sms)) --lg;
-        while (lg > 0 && (line << lg) > kMaxDynSmem) --lg;
-        lg = std::max(0, lg - shift);
-        ap.lg = lg;
-        const int64_t per_sm = (ctas() + sms - 1) / sms;
-        const bool few = per_sm <= 4;
-        const int work = ((few && update ? ap.plan.n : ap.plan.nbmax * fields) << lg) + 31;
-        const int full = c->dtype == PFC_F64 ? kColThreads<double> : kColThreads<float>;
-        const int most = !few ? many : per_sm <= 2 ? (int)(full / per_sm) & ~31 : kGenThreads;
-        ap.threads = std::min(most, std::max(32, work & ~31));
-        ap.smem = ((size_t)ap.plan.np * 16) << lg;
-    };
-    columns(c->py, c->nz, 1, false, o.tile_shift[1]);
-    columns(c->pz, c->ny, 1, false, o.tile_shift[2]);
-    columns(c->pzprop, c->ny, 1, true, o.tile_shift[3]);
-    columns(c->pz2, c->ny, 2, true, o.tile_shift[3]);
-    columns(c->py2, 1, 1, true, o.tile_shift[3]);
-    auto rows = [&](AxisPlan& ap, int work) {  // work: the most items of a line in a stage
-        const int64_t nrows = (int64_t)c->ny * c->nz;
-        int lines = std::max(1, many / work);
-        while (lines > 1 && (nrows + lines * W - 1) / (lines * W) * batch < 2 * (int64_t)sms) lines >>= 1;
-        ap.lines = std::max(1, lines >> o.tile_shift[0]);
-        ap.threads = std::min(kGenThreads, std::max(32, (ap.lines * work + 31) & ~31));
-        ap.smem = (size_t)ap.lines * ap.plan.np * 16;
-    };
-    rows(c->px, c->px.plan.nbmax);
-    if (c->px2.plan.nst) {
-        const GPlan& q = c->px2.plan;
-        int work = q.st[0].m / 2 + 1;
-        for (int i = 1; i < q.nst; ++i) work = std::max(work, q.st[i].nb);
-        rows(c->px2, work);
-    }
-}
 
 pfc_status fail(pfc_ctx* c, pfc_status s, const std::string& msg) {
     if (c) c->err = msg;
@@ -608,33 +432,11 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
     const size_t csz = 2 * c->fsize;
 
     std::vector<std::complex<double>> tab;
-    const bool even = (c->nx % 2) == 0;
-    const int lx = even ? c->nx / 2 : c->nx;
     std::vector<std::complex<double>> gtab;
     std::vector<int> itab;
-    // Radices of the general passes by field size.  Small fields leave most of the GPU idle and
-    // pay for every instruction fetched, so small radices (more threads, less code) win: 256^2
-    // FP64 x pass 5.7 us at radices up to 6, 7.0 at 8 and 10; 600 x 500 FP32 8.0 at 8, 10.0 at
-    // 10; from about a million modes fewer stages win (160 x 150 x 160 FP32 x pass 14.7 at 10,
-    // 17.4 at 8).
-    const int cap = c->n_cmpl < 100000 ? 6 : c->n_cmpl < 1000000 ? 8 : 10;
-    if (!make_plan(lx, c->px.plan, gtab, itab, o.radix_order, cap) ||
-        !make_plan(c->ny, c->py.plan, gtab, itab, o.radix_order, cap) ||
-        !make_plan(c->nz, c->pz.plan, gtab, itab, o.radix_order, cap)) {
+    if (!plan_general(c, o, gtab, itab)) {
         free_ctx(c);
         return PFC_ERR_UNSUPPORTED;
-    }
-    // the paired x pass, where it takes no stage more than the general one (160 x 150 x 160 FP32:
-    // 10 x 8 unpaired 69.5 us per step, 5 x 4 x 4 paired 72)
-    if (!even || !make_plan(lx, c->px2.plan, gtab, itab, o.radix_order, cap, kPairRadix) ||
-        c->px2.plan.nst > c->px.plan.nst)
-        c->px2.plan = GPlan{};
-    c->pzprop.plan = c->pz2.plan = c->pz.plan;
-    c->py2.plan = c->py.plan;
-    c->post_off = (int)gtab.size();
-    for (int k = 0; k <= c->nx / 2; ++k) {
-        const double ang = -2.0 * M_PI * (double)k / (double)c->nx;
-        gtab.emplace_back(std::cos(ang), std::sin(ang));
     }
     auto roots = [&](int n, int count) {
         for (int m = 0; m < count; ++m) {
@@ -731,15 +533,6 @@ pfc_status pfc_create_with(const pfc_desc* d, const pfc_options* opts, pfc_ctx**
         if (cudaGetDevice(&dev) == cudaSuccess)
             cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
         cudaGetLastError();
-    }
-    // lengths whose lines (two of them, padded one element per 32) do not fit a CTA's shared
-    // memory are refused
-    {
-        auto line = [&](int n, int lines) { return (size_t)lines * ((n + (n >> 5) + 1) | 1) * csz; };
-        if (line(lx, 2) > kMaxDynSmem || line(c->ny, 2) > kMaxDynSmem || line(c->nz, 4) > kMaxDynSmem) {
-            free_ctx(c);
-            return PFC_ERR_UNSUPPORTED;
-        }
     }
     plan_launches(c, o, 1, c->num_sms);
     c->n_peak_blocks = peak_chunks(c->nx, c->ny, c->nz);
