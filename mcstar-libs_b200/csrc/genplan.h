@@ -13,15 +13,15 @@ namespace pfc {
 
 // The stages of an n-point plan of the general engine (genfft.cuh), in order.  order 0: the
 // fewest stages with radices up to `cap`, as equal as possible (the least sum), larger
-// radices first; 1: radices up to 5 (4 before 2); 2: as 0 with the odd radices first.  Primes
-// from 7 to kMaxOddRadix are stages of their own.  At least two stages, the last with a
+// radices first; 1: radices up to 5 (4 before 2), and 7; 2: as 0 with the odd radices first.  7 is
+// taken at any cap; primes from 11 to kMaxOddRadix are stages of their own.  At least two stages, the last with a
 // hand-written DFT: a stage of radix 1 is appended where needed.  first > 0: only plans without
 // primes whose smallest radix is at most that, in ascending order.
 inline bool factor_radices(int n, std::vector<int>& rs, int order, int cap, int first) {
     rs.clear();
     if (n < 1) return false;
     std::vector<int> primes;
-    for (int p = 7; p <= kMaxOddRadix; p += 2) {
+    for (int p = 11; p <= kMaxOddRadix; p += 2) {
         bool prime = true;
         for (int d = 3; d * d <= p; d += 2) prime = prime && (p % d != 0);
         if (!prime) continue;
@@ -30,11 +30,11 @@ inline bool factor_radices(int n, std::vector<int>& rs, int order, int cap, int 
     std::vector<int> best;
     if (first > 0 && !primes.empty()) return false;
     if (order == 1) {
-        for (int r : {4, 2, 3, 5})
+        for (int r : {4, 2, 3, 5, 7})
             while (n % r == 0) { best.push_back(r); n /= r; }
         if (n != 1) return false;
     } else {
-        static const int kRadix[] = {10, 9, 8, 6, 5, 4, 3, 2};
+        static const int kRadix[] = {10, 9, 8, 7, 6, 5, 4, 3, 2};
         std::vector<int> cur;
         int best_len = kMaxStages + 1, best_sum = 0;
         // descending factorisations of n; the number of stages bounded by the best so far
@@ -53,7 +53,7 @@ inline bool factor_radices(int n, std::vector<int>& rs, int order, int cap, int 
             }
             if ((int)cur.size() >= best_len) return;
             for (int i = from; i < (int)(sizeof(kRadix) / sizeof(kRadix[0])); ++i)
-                if (rest % kRadix[i] == 0 && kRadix[i] <= cap) {
+                if (rest % kRadix[i] == 0 && (kRadix[i] <= cap || kRadix[i] == 7)) {
                     cur.push_back(kRadix[i]);
                     self(self, rest / kRadix[i], i);
                     cur.pop_back();
@@ -97,6 +97,7 @@ inline bool make_plan(int n, GPlan& p, std::vector<std::complex<double>>& tab, s
         g.m = M / g.R;
         g.nb = n / g.R;
         p.nbmax = std::max(p.nbmax, g.nb);
+        if (g.R > 10) p.nblong = p.nblong ? std::min(p.nblong, g.nb) : g.nb;
         g.ms = s == p.nst - 1 ? 1 : padded(g.m);
         g.Ms = padded(M);
         g.by_m = make_fastdiv(g.m);
@@ -108,13 +109,14 @@ inline bool make_plan(int n, GPlan& p, std::vector<std::complex<double>>& tab, s
                 tab.emplace_back(std::cos(ang), std::sin(ang));
             }
         g.rt = (int)tab.size();
-        if (g.R >= 7 && g.R % 2 && g.R != 9)
+        if (g.R > 10)
             for (int q = 0; q < g.R; ++q) {
                 const double ang = -2.0 * M_PI * (double)q / (double)g.R;
                 tab.emplace_back(std::cos(ang), std::sin(ang));
             }
         M = g.m;
     }
+    if (!p.nblong) p.nblong = p.nbmax;
     // frequency of position q: digits of q by the stages, reversed
     std::vector<int> freq(n);
     for (int q = 0; q < n; ++q) {
@@ -146,7 +148,10 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
     // at most two the SM's whole register file, and an update pass with few CTAs one mode per
     // thread: the update is its longest part (1000^2 FP32 step, 126 CTAs: 46.3 us at 256 threads,
     // 28.3 at 1000; with noise 59.6 and 31.7; two-column tiles at 256 threads 33.4 and 34.0).
-    // Rows: as many as fill those threads.
+    // Rows: as many as fill those threads, by the butterflies of the largest prime radix where there is
+    // one (a 209-point row in FP64 has 11 of radix 19, and by the stage with the most, the appended one of
+    // radix 1, one row per CTA: 209x57x260 x pass 679 us, now
+    // 133).
     const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
     const int many = c->dtype == PFC_F64 ? 128 : 256;
     auto columns = [&](AxisPlan& ap, int64_t planes, int fields, bool update, int shift) {
@@ -170,20 +175,22 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
     columns(c->pzprop, c->ny, 1, true, o.tile_shift[3]);
     columns(c->pz2, c->ny, 2, true, o.tile_shift[3]);
     columns(c->py2, 1, 1, true, o.tile_shift[3]);
-    auto rows = [&](AxisPlan& ap, int work) {  // work: the most items of a line in a stage
+    // work: the most items of a line in a stage; longest: in the stage that takes longest
+    auto rows = [&](AxisPlan& ap, int work, int longest) {
         const int64_t nrows = (int64_t)c->ny * c->nz;
-        int lines = std::max(1, many / work);
+        int lines = std::max(1, many / longest);
+        while (lines > 1 && lines * (size_t)ap.plan.np * 16 > 72 * 1024) lines >>= 1;
         while (lines > 1 && (nrows + lines * W - 1) / (lines * W) * batch < 2 * (int64_t)sms) lines >>= 1;
         ap.lines = std::max(1, lines >> o.tile_shift[0]);
         ap.threads = std::min(kGenThreads, std::max(32, (ap.lines * work + 31) & ~31));
         ap.smem = (size_t)ap.lines * ap.plan.np * 16;
     };
-    rows(c->px, c->px.plan.nbmax);
+    rows(c->px, c->px.plan.nbmax, c->px.plan.nblong);
     if (c->px2.plan.nst) {
         const GPlan& q = c->px2.plan;
         int work = q.st[0].m / 2 + 1;
         for (int i = 1; i < q.nst; ++i) work = std::max(work, q.st[i].nb);
-        rows(c->px2, work);
+        rows(c->px2, work, work);
     }
 }
 
