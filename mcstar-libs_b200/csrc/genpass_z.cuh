@@ -207,6 +207,28 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     });
 }
 
+// The z pass of a slab of a 2D field (nz = 1: the y transforms are the slab's xy part): no transform,
+// so the update of every mode in place, one thread per mode.  (The column pass with lines of one
+// point has a CTA per row and half of its threads idle: 2048 x 1536 FP64 209 us, so 13.)
+template <typename T>
+__global__ void __launch_bounds__(256) k_zflat(cx<T>* A, const cx<T>* B, int nx, int ny, FastDiv by_nxh, ZArgsT<T> a,
+                                               const double2* k0, int* flag) {
+    const int nxh = nx / 2 + 1, m = blockIdx.x * blockDim.x + threadIdx.x;
+    float mc = 0.f;
+    bool bad = false;
+    if (m < nxh * ny) {
+        const int ky = fdiv(m, by_nxh), kx = m - ky * nxh, kyg = ky + a.ky0;
+        const ZColumn<T> col(kx, nx, kwave_ck<T>(kyg, a.nyg, a.cky), a);
+        cx<T> psi = A[m];
+        if (kx == 0 && kyg == 0 && a.prop != kPropRelax && a.prop != kPropRelaxExp) psi = mkc<T>((T)k0->x, (T)k0->y);
+        const cx<T> v = zmode<T>(a.prop, psi, B[m], col, kyg, 0, kwave_ck<T>(0, 1, a.ckz), nx, 1, T(1) + a.C - a.eps, a, mc);
+        bad = !isfinite(v.x) || !isfinite(v.y);
+        A[m] = v;
+    }
+    if ((a.prop == kPropRelax || a.prop == kPropRelaxExp) && a.maxc) fold_max_change(mc, a.maxc);
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
+}
+
 }  // namespace
 
 template <typename T> cudaError_t gen_zattrs() {
@@ -229,6 +251,12 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
     ZArgsT<T> t{(T)a.dt, (T)a.eps, (T)a.C, (T)a.namp_eff, (T)(tp / a.lx), flat ? T(0) : (T)(tp / a.ly),
                 (T)(tp / (flat ? a.ly : a.lz)), a.seed, a.counter, a.dev_counter, a.use_noise, a.final_step, a.prop,
                 a.maxc, a.margs, a.ky0, a.ny_global > 0 ? a.ny_global : ny};
+    if (!flat && !carry && c->nz == 1 && c->batch == 1) {
+        const int modes = c->nxh * c->ny;
+        k_zflat<T><<<(modes + 255) / 256, 256, 0, c->stream>>>((cx<T>*)A, (const cx<T>*)B, c->nx, c->ny,
+                                                               make_fastdiv(c->nxh), t, c->k0, c->flag);
+        return cudaGetLastError();
+    }
     auto k = carry ? k_zprop<T, true> : k_zprop<T, false>;
     return chain_launch(c, k, grid, ap.threads, carry ? ap.smem : 2 * ap.smem, (cx<T>*)A, (const cx<T>*)B, c->nx, ny,
                         ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, t, c->k0, c->flag, c->mstride,

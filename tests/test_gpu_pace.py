@@ -33,3 +33,37 @@ def test_prime_radices(shape, near, dtype):
     """A radix of 7 to 31 costs (R + 1) / 2 products per point where 2-3-5 stages cost about 2 to 3
     (measured ratios 1.6 to 2.6; with the points loaded and multiplied out one by one 12 to 24)."""
     assert step_time(shape, dtype) < 7 * step_time(near, dtype)
+
+
+def event_time(f, n=20):
+    import torch
+    f()
+    torch.cuda.synchronize()
+    best = math.inf
+    for _ in range(5):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        for _ in range(n):
+            f()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) / n)
+    return best
+
+
+@pytest.mark.parametrize("dtype", [F32, F64], ids=["f32", "f64"])
+def test_flat_slab_update(dtype):
+    """The z pass of a 2D slab is an update of every mode, as pfc_update_eom is (as a column pass with
+    lines of one point it took 6 to 8 times that)."""
+    import ctypes
+    from mcstar_b200 import Context
+    from mcstar_b200._lib import PfcStepParams
+    ctx = Context((2048, 1536, 1), dtype)
+    a, b = ctx.empty_state(), ctx.empty_state()
+    a.zero_()
+    b.zero_()
+    lens = (1600.0, 1200.0, 1.0)
+    p = PfcStepParams(0.25, 0.3, 0.0, 1.0, 0.0, *lens, 3, 0)
+    flat = event_time(lambda: ctx._call("pfc_slab_zpass", ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(b.data_ptr()),
+                                        ctypes.byref(p), 0, 1536, 0))
+    assert flat < 2.5 * event_time(lambda: ctx.update_eom(a, b, None, 0.0, 0.25, 0.3, lens))
