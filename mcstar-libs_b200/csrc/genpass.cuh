@@ -30,13 +30,14 @@ template <typename T> constexpr int kColThreads = sizeof(T) == 8 ? 768 : 1024;
 // largest first radix of the stepper's paired x pass (two butterflies in registers)
 constexpr int kPairRadix = 5;
 
-// The columns of a CTA: 2^lg elements of one column (FP64) or of two columns 2^lg apart (FP32;
-// consecutive threads then move consecutive columns of either half), from column i0 of ni.
+// The columns of a CTA: 2^lg elements of one column (FP64, and FP32 with w = 1: the second line
+// then holds zeros) or of two columns 2^lg apart (FP32, w = 2; consecutive threads then move
+// consecutive columns of either half), of ni.
 template <typename T> struct ColTile {
     int i0, n, second;
-    __device__ __forceinline__ ColTile(int lg, int ni, int col0 = 0) {
-        i0 = col0 + blockIdx.x * (Elem<T>::lines << lg);
-        n = ni - i0;
+    __device__ __forceinline__ ColTile(int lg, int w, int ni) {
+        i0 = blockIdx.x * (w << lg);
+        n = min(ni - i0, w << lg);
         second = 1 << lg;
     }
     __device__ __forceinline__ bool ok(int i, int half) const { return i + half * second < n; }

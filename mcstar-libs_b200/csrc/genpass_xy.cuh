@@ -9,21 +9,22 @@ namespace {
 
 // ---------------------------------------------------------------------------------
 // complex FFT along a strided axis: element (line o, inner i, position k) at
-// base + o*os + i + k*es.  A CTA owns 2^lg elements (FP64: lines,
-// FP32: pairs of lines) of consecutive inner lines of one o.  Forward
+// base + o*os + i + k*es.  A CTA owns 2^lg elements of w consecutive inner lines each (FP64:
+// w = 1, FP32: 1 or 2) of one o.  Forward
 // transforms run down from natural order, inverse ones up to it: the inverse is then, bit
 // for bit, the one of the stepper's z pass (k_zprop).
 // ---------------------------------------------------------------------------------
 template <typename T, int DIR>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_cols(const cx<T>* in, cx<T>* out, int ni, int64_t es, int64_t os, const __grid_constant__ GPlan p,
-           const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, double scale, int64_t ms) {
+           const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, int w, double scale,
+           int64_t ms) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
     chain_start();
     chain_wait();
     const ColLines lay{lg};
-    const ColTile<T> tile{lg, ni};
+    const ColTile<T> tile{lg, w, ni};
     const int64_t base = (int64_t)blockIdx.y * os + tile.i0 + blockIdx.z * ms;  // grid z: fields of a batch
     in += base;
     out += base;
@@ -85,21 +86,21 @@ __device__ __forceinline__ R cubic(R v, R mul, R nC, R nmu) {  // nC = -C, nmu =
 // kR2C: real rows (in) to half-spectrum rows (out); kC2R: half-spectrum rows to real rows;
 // kNonlin: the stepper's x pass, C2R, the cubic nonlinearity, R2C, in place on rows of the
 // mixed (kx, y, z) field (in == out).  A CTA owns rpc lines of
-// the engine: whole rows (FP64) or pairs of rows (FP32).  The transforms leave
+// the engine: whole rows (W = 1; FP32: each twice) or pairs of rows (FP32, W = 2).  The transforms leave
 // frequencies (or cells) digit-reversed; the R2C merge and the C2R output read them back in
 // natural order through the position table, so that global accesses stay contiguous.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
     k_rows(const void* in, void* out, int nrows, int nx, const __grid_constant__ GPlan p,
            const el<T>* __restrict__ tw, const int* __restrict__ tab, const el<T>* __restrict__ post, int rpc,
-           double mul, double C, double mu, int64_t ms, FastDiv by_nxh) {
+           int W, double mul, double C, double mu, int64_t ms, FastDiv by_nxh) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
     chain_start();
     chain_wait();
-    constexpr int W = Elem<T>::lines;
+    if (Elem<T>::lines == 1) W = 1;
     const int row0 = blockIdx.x * rpc * W;
-    const int nr = min(rpc * W, nrows - row0), nl = (nr + W - 1) / W;
+    const int nr = min(rpc * W, nrows - row0), nl = W > 1 ? (nr + 1) / 2 : nr;
     const RowLines lay{nl, p.np};
     const int L = p.n, nxh = nx / 2 + 1;
     const bool even = (nx & 1) == 0;
@@ -228,16 +229,17 @@ template <class F> __device__ __forceinline__ void by_pair_radix(int R, F&& f) {
 template <typename T>
 __global__ void __launch_bounds__(kGenThreads, 3)
     k_xpass(cx<T>* field, int nrows, int nxh, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
-            const el<T>* __restrict__ post, int rpc, FastDiv by_half, double mul, double C, double mu, int64_t ms) {
+            const el<T>* __restrict__ post, int rpc, int W, FastDiv by_half, double mul, double C, double mu,
+            int64_t ms) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
     chain_start();
     chain_wait();
     using E = Elem<T>;
     using CC = CE<T>;
-    constexpr int W = E::lines;
+    if (E::lines == 1) W = 1;
     const int row0 = blockIdx.x * rpc * W;
-    const int nr = min(rpc * W, nrows - row0), nl = (nr + W - 1) / W;
+    const int nr = min(rpc * W, nrows - row0), nl = W > 1 ? (nr + 1) / 2 : nr;
     const RowLines lay{nl, p.np};
     const int L = p.n;
     const GStage& s0 = p.st[0];
@@ -373,11 +375,11 @@ cudaError_t gen_cols(const pfc_ctx* c, int axis, int dir, const void* in, void* 
     int no;
     if (axis == 1) { es = c->nxh; os = (int64_t)c->ny * c->nxh; no = c->nz; }
     else { es = (int64_t)c->ny * c->nxh; os = c->nxh; no = c->ny; }
-    const int tile = Elem<T>::lines << ap.lg;
+    const int tile = ap.w << ap.lg;
     dim3 grid((c->nxh + tile - 1) / tile, no, c->batch);
     auto k = dir < 0 ? k_cols<T, -1> : k_cols<T, 1>;
     return chain_launch(c, k, grid, ap.threads, ap.smem, (const cx<T>*)in, (cx<T>*)out, c->nxh, es, os, ap.plan,
-                        (const el<T>*)c->gtw, c->fft_tab, ap.lg, scale, c->mstride);
+                        (const el<T>*)c->gtw, c->fft_tab, ap.lg, ap.w, scale, c->mstride);
 }
 
 template <typename T>
@@ -386,18 +388,18 @@ cudaError_t gen_rows(const pfc_ctx* c, int mode, const void* in, void* out, doub
     if (mode == kNonlin && c->px2.plan.nst) {
         const AxisPlan& ap = c->px2;
         const el<T>* tw = (const el<T>*)c->gtw;
-        const int rows = ap.lines * Elem<T>::lines;
+        const int rows = ap.lines * ap.w;
         return chain_launch(c, k_xpass<T>, dim3((nrows + rows - 1) / rows, 1, c->batch), ap.threads, ap.smem,
-                            (cx<T>*)out, nrows, c->nxh, ap.plan, tw, tw + c->post_off, ap.lines,
+                            (cx<T>*)out, nrows, c->nxh, ap.plan, tw, tw + c->post_off, ap.lines, ap.w,
                             make_fastdiv(ap.plan.st[0].m / 2 + 1), mul, C, mu, c->mstride);
     }
     const AxisPlan& ap = c->px;
     const el<T>* tw = (const el<T>*)c->gtw;
-    const int rows = ap.lines * Elem<T>::lines;
+    const int rows = ap.lines * ap.w;
     // (the plain transforms run on one field; the x pass on all fields of a batch)
     dim3 grid((nrows + rows - 1) / rows, 1, mode == kNonlin ? c->batch : 1);
     auto k = mode == kR2C ? k_rows<T, kR2C> : mode == kC2R ? k_rows<T, kC2R> : k_rows<T, kNonlin>;
     return chain_launch(c, k, grid, ap.threads, ap.smem, in, out, nrows, c->nx, ap.plan, tw, c->fft_tab,
-                        tw + c->post_off, ap.lines, mul, C, mu, c->mstride, make_fastdiv(c->nxh));
+                        tw + c->post_off, ap.lines, ap.w, mul, C, mu, c->mstride, make_fastdiv(c->nxh));
 }
 }  // namespace pfc

@@ -116,7 +116,7 @@ __device__ __forceinline__ cx<T> zmode(int prop, A&&... args) {
 template <typename T, bool CARRY>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_zprop(cx<T>* A, const cx<T>* B, int nx, int ny, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
-            const int* __restrict__ tab, int lg, ZArgsT<T> a, const double2* k0, int* flag, int64_t ms,
+            const int* __restrict__ tab, int lg, int w, ZArgsT<T> a, const double2* k0, int* flag, int64_t ms,
             cx<T>* anext) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     chain_wait();
     zmember(a);
     const int nxh = nx / 2 + 1, n = p.n;
-    const ColTile<T> tile{lg, nxh};
+    const ColTile<T> tile{lg, w, nxh};
     const int i0 = tile.i0, ky = blockIdx.y;
     const int64_t es = (int64_t)ny * nxh;
     const int64_t base = blockIdx.z * ms + (int64_t)ky * nxh + i0;  // grid z: fields of a batch
@@ -245,7 +245,7 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
                       bool flat) {
     if (a.prop == kPropConservedHpfc && !flat) return cudaErrorNotSupported;
     const AxisPlan& ap = flat ? c->py2 : carry ? c->pzprop : c->pz2;
-    const int ny = flat ? 1 : c->ny, tile = Elem<T>::lines << ap.lg;
+    const int ny = flat ? 1 : c->ny, tile = ap.w << ap.lg;
     const double tp = 6.283185307179586232;
     dim3 grid((c->nxh + tile - 1) / tile, ny, c->batch);
     ZArgsT<T> t{(T)a.dt, (T)a.eps, (T)a.C, (T)a.namp_eff, (T)(tp / a.lx), flat ? T(0) : (T)(tp / a.ly),
@@ -259,7 +259,7 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
     }
     auto k = carry ? k_zprop<T, true> : k_zprop<T, false>;
     return chain_launch(c, k, grid, ap.threads, carry ? ap.smem : 2 * ap.smem, (cx<T>*)A, (const cx<T>*)B, c->nx, ny,
-                        ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, t, c->k0, c->flag, c->mstride,
+                        ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, ap.w, t, c->k0, c->flag, c->mstride,
                         (cx<T>*)anext);
 }
 

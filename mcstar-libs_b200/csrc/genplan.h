@@ -143,32 +143,47 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
     // Columns: 128-byte segments (8 elements of 16 bytes:
     // 16 FP32 or 8 FP64 columns), halved down to the 32-byte sectors of L2 while the tile's
     // shared memory would leave fewer than three CTAs per SM, or the pass fewer than two CTAs
-    // per SM; then tile_shift times.  Threads: one butterfly each in the stage with the most, up
-    // to 256 (FP64: 128, for more CTAs per SM); a pass with at most four CTAs per SM takes 256, with
-    // at most two the SM's whole register file, and an update pass with few CTAs one mode per
-    // thread: the update is its longest part (1000^2 FP32 step, 126 CTAs: 46.3 us at 256 threads,
-    // 28.3 at 1000; with noise 59.6 and 31.7; two-column tiles at 256 threads 33.4 and 34.0).
+    // per SM; on down to one column while that gives no more than a CTA per SM and an eighth: a
+    // pass with so few CTAs takes as long as one of them, whatever it wastes.  y columns and update
+    // of FP32 fields, us at 4, 2 and 1 columns: 64 x 2048 (33 columns) 15.8, 11.6, 9.7 and 37.6,
+    // 25.4, 20.9; 256 x 1500 (129) 10.3, 8.1, 7.2 and 26.4, 19.6, 16.6; 300 x 300 (151) 4.9, 4.8, 4.8
+    // and 11.5, 10.7, 10.0; 1000 x 1000 (501) 8.0, 8.9, 10.8 and 20.1, 21.4, 29.9.  Then tile_shift
+    // times.  Threads: one butterfly each in the stage with the most, up to 256 (FP64: 128, for
+    // more CTAs per SM); a pass with at most four CTAs per SM takes 256, with at most two the SM's
+    // whole register file, and an update pass with few CTAs one mode per thread: the update is its
+    // longest part (1000^2 FP32 step, 126 CTAs: 46.3 us at 256 threads, 28.3 at 1000; with noise 59.6
+    // and 31.7; two-column tiles at 256 threads 33.4 and 34.0).
     // Rows: as many as fill those threads, by the butterflies of the largest prime radix where there is
     // one (a 209-point row in FP64 has 11 of radix 19, and by the stage with the most, the appended one of
-    // radix 1, one row per CTA: 209x57x260 x pass 679 us, now
-    // 133).
+    // radix 1, one row per CTA: 209x57x260 x pass 679 us, now 133).  With at most four CTAs per SM
+    // at least a thread for two points, for the loops over the row's modes (1024 x 240 FP32, two
+    // rows: C2R rows 10.6 us at 64 threads, 9.0 at 256; 128 x 45 x 30, eight rows: R2C 5.1 at 64,
+    // 4.4 at 256).
     const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
     const int many = c->dtype == PFC_F64 ? 128 : 256;
     auto columns = [&](AxisPlan& ap, int64_t planes, int fields, bool update, int shift) {
         const size_t line = (size_t)ap.plan.np * 16 * fields;
-        int lg = 3;
-        auto ctas = [&] { return ((c->nxh + (W << lg) - 1) / (W << lg)) * planes * batch; };
-        while (lg > 1 && ((line << lg) > 72 * 1024 || ctas() < 2 * (int64_t)sms)) --lg;
-        while (lg > 0 && (line << lg) > kMaxDynSmem) --lg;
-        lg = std::max(0, lg - shift);
-        ap.lg = lg;
+        int cols = 8 * W;  // columns of a CTA
+        auto shape = [&](int n) {
+            cols = n;
+            ap.w = std::min(W, n);
+            ap.lg = 0;
+            while ((ap.w << ap.lg) < n) ++ap.lg;
+        };
+        auto ctas = [&] { return (c->nxh + cols - 1) / cols * planes * batch; };
+        auto bytes = [&] { return line * (size_t)std::max(1, cols / W); };
+        while (cols > 2 && cols / 2 >= c->nxh) cols /= 2;
+        while (cols > 2 * W && (bytes() > 72 * 1024 || ctas() < 2 * (int64_t)sms)) cols /= 2;
+        while (cols > 1 && (c->nxh + cols / 2 - 1) / (cols / 2) * planes * batch <= sms + sms / 8) cols /= 2;
+        while (cols > W && bytes() > kMaxDynSmem) cols /= 2;
+        shape(std::max(1, cols >> shift));
         const int64_t per_sm = (ctas() + sms - 1) / sms;
         const bool few = per_sm <= 4;
-        const int work = ((few && update ? ap.plan.n : ap.plan.nbmax * fields) << lg) + 31;
+        const int work = ((few && update ? ap.plan.n : ap.plan.nbmax * fields) << ap.lg) + 31;
         const int full = c->dtype == PFC_F64 ? kColThreads<double> : kColThreads<float>;
         const int most = !few ? many : per_sm <= 2 ? (int)(full / per_sm) & ~31 : kGenThreads;
         ap.threads = std::min(most, std::max(32, work & ~31));
-        ap.smem = ((size_t)ap.plan.np * 16) << lg;
+        ap.smem = ((size_t)ap.plan.np * 16) << ap.lg;
     };
     columns(c->py, c->nz, 1, false, o.tile_shift[1]);
     columns(c->pz, c->ny, 1, false, o.tile_shift[2]);
@@ -178,11 +193,16 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
     // work: the most items of a line in a stage; longest: in the stage that takes longest
     auto rows = [&](AxisPlan& ap, int work, int longest) {
         const int64_t nrows = (int64_t)c->ny * c->nz;
-        int lines = std::max(1, many / longest);
-        while (lines > 1 && lines * (size_t)ap.plan.np * 16 > 72 * 1024) lines >>= 1;
-        while (lines > 1 && (nrows + lines * W - 1) / (lines * W) * batch < 2 * (int64_t)sms) lines >>= 1;
-        ap.lines = std::max(1, lines >> o.tile_shift[0]);
-        ap.threads = std::min(kGenThreads, std::max(32, (ap.lines * work + 31) & ~31));
+        int rpc = std::max(1, many / longest) * W;  // rows of a CTA
+        auto bytes = [&] { return (size_t)(rpc / W) * ap.plan.np * 16; };
+        while (rpc > W && bytes() > 72 * 1024) rpc = rpc / (2 * W) * W;
+        while (rpc > W && (nrows + rpc - 1) / rpc * batch < 2 * (int64_t)sms) rpc = rpc / (2 * W) * W;
+        for (int i = 0; i < o.tile_shift[0] && rpc > 1; ++i) rpc = rpc > W ? rpc / (2 * W) * W : 1;
+        ap.w = std::min(W, rpc);
+        ap.lines = rpc / ap.w;
+        int items = ap.lines * work;
+        if ((nrows + rpc - 1) / rpc * batch <= 4 * (int64_t)sms) items = std::max(items, ap.lines * ap.plan.n / 2);
+        ap.threads = std::min(kGenThreads, std::max(32, (items + 31) & ~31));
         ap.smem = (size_t)ap.lines * ap.plan.np * 16;
     };
     rows(c->px, c->px.plan.nbmax, c->px.plan.nblong);

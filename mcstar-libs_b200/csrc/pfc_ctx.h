@@ -18,8 +18,9 @@ constexpr int kPeakBlock = 256;         // cells per block of the peak finder
 
 struct AxisPlan {
     GPlan plan;
-    int lg;            // 2^lg elements per position and CTA (y, z): columns, in FP32 pairs of columns
-    int lines;         // engine lines per CTA (x): rows, in FP32 pairs of rows
+    int w;             // lines (columns, rows) of an element: 1, in FP32 1 or 2
+    int lg;            // 2^lg elements per position and CTA (y, z)
+    int lines;         // elements of lines per CTA (x)
     int threads;
     size_t smem;       // dynamic shared memory of the CTA's lines
 };
