@@ -18,10 +18,10 @@ template <typename T, int DIR>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_cols(const cx<T>* in, cx<T>* out, int ni, int64_t es, int64_t os, const __grid_constant__ GPlan p,
            const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, int w, double scale,
-           int64_t ms) {
+           int64_t ms, int lead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
-    chain_start();
+    chain_start(lead);
     chain_wait();
     const ColLines lay{lg};
     const ColTile<T> tile{lg, w, ni};
@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
                             [&](int i, int j, int m) { return tile.get(in + i + j * es, i, m * es); });
         __syncthreads();
         stages_mid<T, DIR>(buf, p, lay, tw);
+        chain_start();
         stage_last<T, DIR>(buf, p, lay, tw, tab + p.rev,
                            [&](int i, int k0) { return put(out + i + k0 * es, i, p.kstep * es); });
     } else {
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
                          [&](int i, int k0) { return tile.get(in + i + k0 * es, i, p.kstep * es); });
         __syncthreads();
         stages_back<T, DIR>(buf, p, lay, tw);
+        chain_start();
         stage_out<T, DIR>(buf, p, lay, tw,
                           [&](int i, int j, int m) { return put(out + i + j * es, i, m * es); });
     }
@@ -93,10 +95,10 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
     k_rows(const void* in, void* out, int nrows, int nx, const __grid_constant__ GPlan p,
            const el<T>* __restrict__ tw, const int* __restrict__ tab, const el<T>* __restrict__ post, int rpc,
-           int W, double mul, double C, double mu, int64_t ms, FastDiv by_nxh) {
+           int W, double mul, double C, double mu, int64_t ms, FastDiv by_nxh, int lead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
-    chain_start();
+    chain_start(lead);
     chain_wait();
     if (Elem<T>::lines == 1) W = 1;
     const int row0 = blockIdx.x * rpc * W;
@@ -143,6 +145,7 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
     if (MODE == kC2R) {
         stage_inplace<T, 1, false, false>(buf, p, p.nst - 1, lay, tw);
         __syncthreads();
+        chain_start();
         T* rows = static_cast<T*>(out) + (int64_t)row0 * nx;
         for (int e = threadIdx.x; e < nl * L; e += blockDim.x) {
             const int i = fdiv(e, p.by_n), m = e - i * L;
@@ -189,6 +192,7 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
         stage_inplace<T, -1, true, true>(buf, p, 0, lay, tw);
         __syncthreads();
     }
+    chain_start();
     // the merge, in the order of the frequencies: natural after the transform back (kNonlin),
     // through the position table otherwise
     cx<T>* rows = static_cast<cx<T>*>(out) + blockIdx.z * ms + (int64_t)row0 * nxh;
@@ -230,10 +234,10 @@ template <typename T>
 __global__ void __launch_bounds__(kGenThreads, 3)
     k_xpass(cx<T>* field, int nrows, int nxh, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
             const el<T>* __restrict__ post, int rpc, int W, FastDiv by_half, double mul, double C, double mu,
-            int64_t ms) {
+            int64_t ms, int lead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
-    chain_start();
+    chain_start(lead);
     chain_wait();
     using E = Elem<T>;
     using CC = CE<T>;
@@ -305,6 +309,7 @@ __global__ void __launch_bounds__(kGenThreads, 3)
     }
     __syncthreads();
     stages_back<T, -1>(buf, p, lay, tw);
+    chain_start();
     by_pair_radix(s0.R, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         for (int e = threadIdx.x; e < total; e += blockDim.x) {

@@ -117,10 +117,10 @@ template <typename T, bool CARRY>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_zprop(cx<T>* A, const cx<T>* B, int nx, int ny, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
             const int* __restrict__ tab, int lg, int w, ZArgsT<T> a, const double2* k0, int* flag, int64_t ms,
-            cx<T>* anext) {
+            cx<T>* anext, int lead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
-    chain_start();
+    chain_start(lead);
     chain_wait();
     zmember(a);
     const int nxh = nx / 2 + 1, n = p.n;
@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     stage_inplace<T, 1, true, false>(buf, p, p.nst - 1, lay, tw);
     __syncthreads();
     stages_back<T, 1>(buf, p, lay, tw);
+    chain_start();
     cx<T>* dst = CARRY ? anext + base : A;
     // (the entry transform's scale, so that a resumed run repeats the bits)
     const typename Elem<T>::real scale = Elem<T>::bc(1.0 / (double)n);

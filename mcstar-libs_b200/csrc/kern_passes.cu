@@ -44,7 +44,7 @@ struct YCfg {
 template <class Y, int DIR, bool kZ>
 __global__ void __launch_bounds__(Y::T, Y::MINB)
     k_ycol(const float2* in, float2* out, int nxh, int ny, int nz, int lay, const float2* __restrict__ twg,
-           float scale, int64_t ms, int q0, float2* copy) {
+           float scale, int64_t ms, int q0, float2* copy, int lead) {
     // the columns of NY elements of kx tile blockIdx.x at plane q0 + blockIdx.y: y columns of
     // that z-plane (kZ false) or z columns at that ky (kZ); lay & 3: the layout of the input,
     // lay >> 2: of the output (col_addr).  With the standard layout on both sides, in may
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(Y::T, Y::MINB)
     float2* xb = sm;
     float2* tw = sm + Y::XB;
     const int tid = threadIdx.x;
-    chain_start();
+    chain_start(lead);
     for (int i = tid; i < NY; i += Y::T) tw[i] = twg[i];
     chain_wait();
     const int c = tid % TX, t = tid / TX;
@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(Y::T, Y::MINB)
     }
     __syncthreads();
     fft_d1_to_d2<NY, E, TX, DIR, BarCta, Y::PADG>(v, t, c, xb, tw);
+    chain_start();
     if (valid) {
         const ColAddr ao = col_addr(lay >> 2, kZ, kx, q, nxh, ny, nz);
 #pragma unroll
@@ -329,7 +330,7 @@ __device__ __forceinline__ void row_tiles_r2c(const float2* rb, const float2* tw
 template <class X, int MODE>
 __global__ void __launch_bounds__(X::T, X::MINB)
     k_xrow(const float2* in, float2* out, const float* pot, int nrows, const float2* __restrict__ twg,
-           float mul, float Cc, float mu, int64_t ms) {
+           float mul, float Cc, float mu, int64_t ms, int lead) {
     constexpr int NX = X::NX, M = X::M, NXH = X::NXH, E = X::E, P = X::P, U = X::U, R = X::R, LDR = X::LDR;
     in += blockIdx.z * ms;  // fields of a batch (grid z; no potential then)
     out += blockIdx.z * ms;
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(X::T, X::MINB)
     float2* twM = sm + X::BUF;  // W_M^m, m < M
     float2* twP = twM + M;      // W_NX^k, k <= M
     const int tid = threadIdx.x;
-    chain_start();
+    chain_start(lead);
     for (int i = tid; i < 2 * M + 1; i += X::T) twM[i] = twg[i];
     chain_wait();
     const int r = tid % R, t = tid / R;
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(X::T, X::MINB)
     }
     if constexpr (MODE == 2) {
         // real pairs out through shared memory, so that rows are stored contiguously
+        chain_start();
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -398,6 +400,7 @@ __global__ void __launch_bounds__(X::T, X::MINB)
             }
     }
     fft_d2_to_d1<M, E, R, -1>(v, t, r, rb, twM);
+    chain_start();
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < E; ++j) rb[r * LDR + t + P * j] = v[j];

@@ -229,7 +229,7 @@ __device__ __forceinline__ void store_state(float2 (&v)[Z::E], float2* A, int64_
 template <class Z, int PROP>
 __global__ void __launch_bounds__(Z::T, Z::MINB) k_zcol(const float2* A, const float2* B, float2* O,
                                                    int nx, int ny, int lay, ZArgsF a, const double2* k0, int* flag,
-                                                   const float2* __restrict__ twg, int64_t ms) {
+                                                   const float2* __restrict__ twg, int64_t ms, int lead) {
     constexpr int NZ = Z::NZ, E = Z::E, TX = Z::TX, P = Z::P, U = Z::U, TH = Z::TH;
     A += blockIdx.z * ms;  // fields of a batch (grid z)
     B += blockIdx.z * ms;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(Z::T, Z::MINB) k_zcol(const float2* A, const f
     float2* regB = sm + Z::REG;
     float2* tw = sm + 2 * Z::REG;
     const int tid = threadIdx.x;
-    chain_start();
+    chain_start(lead);
     const float* kz_tab = load_tail<Z>(tw, twg, a, tid, Z::T);
     chain_wait();
     const int half = tid / TH;
@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(Z::T, Z::MINB) k_zcol(const float2* A, const f
     }
     if (!a.final_step) fft_d2_to_d1<NZ, E, TX, 1, BarDyn, Z::PADG>(v, t, c, regA, tw, bar);
     watch<Z>(v, a.final_step, valid, flag);
+    chain_start();
     const ColAddr co = col_addr((lay & 4) ? 1 : 0, true, kx, ky, nxh, ny, NZ);
     store_state<Z>(v, O, co.base, co.stride, t, valid, a.final_step);
 }
@@ -485,7 +486,7 @@ __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_grou
 template <class Z, int PROP>
 __global__ void __launch_bounds__(Z::TH, Z::CMINB) k_zcarry(float2* kpsi, float2* A, const float2* B, int nx,
                                                       int ny, ZArgsF a, const double2* k0, int* flag,
-                                                      const float2* __restrict__ twg, int64_t ms) {
+                                                      const float2* __restrict__ twg, int64_t ms, int lead) {
     constexpr int NZ = Z::NZ, E = Z::E, TX = Z::TX, P = Z::P, TH = Z::TH;
     static_assert(TX == 8 && (Z::U == 1 || Z::U == 2), "staging swizzle assumes 8 columns per tile");
     kpsi += blockIdx.z * ms;  // fields of a batch (grid z)
@@ -505,7 +506,7 @@ __global__ void __launch_bounds__(Z::TH, Z::CMINB) k_zcarry(float2* kpsi, float2
     const bool valid = kx < nxh;  // the last tile holds only the kx = nx/2 column
     const int64_t zs = (int64_t)ny * nxh;
     const int64_t base = (int64_t)ky * nxh + kx;
-    chain_start();
+    chain_start(lead);
     chain_wait();
     if (valid) {
 #pragma unroll 4
@@ -532,6 +533,7 @@ __global__ void __launch_bounds__(Z::TH, Z::CMINB) k_zcarry(float2* kpsi, float2
     if (a.final_step) return;
     fft_d2_to_d1<NZ, E, TX, 1, BarCta, Z::PADG>(v, t, c, xb, tw);
     watch<Z>(v, false, valid, flag);
+    chain_start();
     store_state<Z>(v, A, base, zs, t, valid, false);
 }
 
