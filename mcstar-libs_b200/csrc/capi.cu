@@ -921,6 +921,7 @@ pfc_status pfc_step_host(pfc_ctx* ctx, const void* host_in, void* host_out, void
 pfc_status pfc_slab_zinv(pfc_ctx* ctx, const void* kpsi, void* A, int ky0) {
     PFC_CHECK_CTX();
     if (!kpsi || !A || kpsi == A || ky0 < 0) return fail(ctx, PFC_ERR_INVALID, "pfc_slab_zinv: bad arguments");
+    const ChainScope chained(ctx);
     if (ky0 == 0) PFC_CUDA(launch_k0_save(ctx, kpsi), "pfc_slab_zinv k0");
     if (ctx->nz > 1) {
         PFC_CUDA(zcols(ctx, 1, kpsi, A, 1.0 / ctx->nz), "pfc_slab_zinv");
@@ -933,6 +934,7 @@ pfc_status pfc_slab_zinv(pfc_ctx* ctx, const void* kpsi, void* A, int ky0) {
 pfc_status pfc_slab_xy(pfc_ctx* ctx, const void* A, void* B, double C, double mu) {
     PFC_CHECK_CTX();
     if (!A || !B || A == B) return fail(ctx, PFC_ERR_INVALID, "pfc_slab_xy: bad arguments");
+    const ChainScope chained(ctx);
     const double mul = 1.0 / ((double)ctx->nx * (double)ctx->ny);
     if (ctx->xy_mode == 2) {
         PFC_CUDA(launch_ypass(ctx, 1, A, B, 1.0, ctx->nz), "pfc_slab_xy y");
@@ -953,6 +955,7 @@ pfc_status pfc_slab_zpass(pfc_ctx* ctx, void* A, const void* B, const pfc_step_p
     PFC_CHECK_CTX();
     if (!A || !B || !p || ky0 < 0 || ny_global < ctx->ny || ky0 + ctx->ny > ny_global)
         return fail(ctx, PFC_ERR_INVALID, "pfc_slab_zpass: bad arguments");
+    const ChainScope chained(ctx);
     ZPropArgs za = zargs(ctx, p);
     // the noise amplitude of the whole field: sqrt(N) of its nx ny_global nz cells
     za.namp_eff = p->namp * std::sqrt((double)ctx->nx * (double)ny_global * (double)ctx->nz);
