@@ -232,12 +232,14 @@ cudaError_t step_exit(pfc_ctx* ctx, void* kpsi) {
 cudaError_t step_xy(pfc_ctx* ctx, void* kpsi, const pfc_step_params* p, bool last) {
     const void* A = carried_A(ctx, kpsi);
     void* B = ctx->work;
+    const double mul = 1.0 / ((double)ctx->nx * (double)ctx->ny);
     if (ctx->nz == 1)  // 2D: the rows of A in place (the y transforms are the update pass's)
         return traced(ctx, 1, 1, [&] {
-            if (ctx->xy_mode == 2) return launch_xpass(ctx, B, nullptr, 1.0 / ctx->nx, p->C, p->mu, 1);
-            return launch_rows_nonlin(ctx, B, 1.0 / ctx->nx, p->C, p->mu);
+            // A holds the factor 1/ny, rounded: the rest, so that the product is off by one rounding
+            const double inv = 1.0 / ctx->ny, rest = mul / (ctx->dtype == PFC_F64 ? inv : (double)(float)inv);
+            if (ctx->xy_mode == 2) return launch_xpass(ctx, B, nullptr, rest, p->C, p->mu, 1);
+            return launch_rows_nonlin(ctx, B, rest, p->C, p->mu);
         });
-    const double mul = 1.0 / ((double)ctx->nx * (double)ctx->ny);
     if (ctx->tiled) {
         void* R = row_field(ctx, kpsi);
         void* Bt = ctx->z_carry ? ctx->work : kpsi;

@@ -12,9 +12,22 @@ namespace {
 // forward transform of the nonlinear term, the semi-implicit update (eom.hpp:60-72 with
 // stabilisation C) with its noise, and the inverse transform for the next step.
 // ---------------------------------------------------------------------------------
+// 2 pi / L of an axis, in FP32 with its rounding: that is the same for all modes of the axis, and grows
+// into the state step by step
+template <typename T> struct Wave {
+    T hi, lo;
+    explicit Wave(double k) : hi((T)k), lo((T)(k - (double)(T)k)) {}
+    // the wavenumber of index i of n (common.hpp:27-28)
+    __device__ __forceinline__ T at(int i, int n) const {
+        const T m = T(i < n / 2 + 1 ? i : i - n);
+        return sizeof(T) == 4 ? fma(m, lo, m * hi) : m * hi;
+    }
+};
+
 template <typename T>
 struct ZArgsT {
-    T dt, eps, C, namp_eff, ckx, cky, ckz;  // ck = 2 pi / L per axis
+    T dt, eps, C, namp_eff;
+    Wave<T> ckx, cky, ckz;
     uint64_t seed, counter;
     const unsigned long long* dev_counter;  // read instead of counter when set
     int use_noise, final_step, prop;
@@ -40,17 +53,8 @@ template <typename T> struct ZColumn {
     int kx;
     T kk0, kxy;
     __device__ __forceinline__ ZColumn(int kx_, int nx, T k1, const ZArgsT<T>& a)
-        : kx(kx_), kk0(kwave_ck<T>(kx_, nx, a.ckx)), kxy(kk0 * kk0 + k1 * k1) {}
+        : kx(kx_), kk0(a.ckx.at(kx_, nx)), kxy(kk0 * kk0 + k1 * k1) {}
 };
-
-// 1 / d: in FP32 the approximate reciprocal and one Newton step (within an ulp) in place of the
-// division's dozen instructions. Where the step has no number (d zero, infinite or NaN: a D that
-// overflowed, or bad parameters) the approximation stands, which is the division's value.
-__device__ __forceinline__ float recip(float d) {
-    const float r = __fdividef(1.0f, d), e = fmaf(-d, r, 1.0f);
-    return e == e ? fmaf(r, e, r) : r;
-}
-__device__ __forceinline__ double recip(double d) { return 1.0 / d; }
 
 // The update of mode (kx, kyg, kz) from psi^ and N^ by propagator PROP with its noise; kk2 =
 // the kz wavenumber, deps = 1 + C - eps.  At k = 0 the conserved propagators return psi^
@@ -63,7 +67,7 @@ __device__ __forceinline__ cx<T> zmode_of(cx<T> psi, cx<T> nl, const ZColumn<T>&
     cx<T> v;
     if constexpr (PROP == kPropConserved) {
         const T dopy = dopx * dopx;
-        const T inv = recip(T(1) - a.dt * (deps * dopx + T(2) * dopy + dopx * dopy));
+        const T denom = T(1) - a.dt * (deps * dopx + T(2) * dopy + dopx * dopy);
         const T f = a.dt * dopx;
         cx<T> num = mkc<T>(psi.x + f * nl.x, psi.y + f * nl.y);
         if (a.use_noise) {
@@ -72,7 +76,7 @@ __device__ __forceinline__ cx<T> zmode_of(cx<T> psi, cx<T> nl, const ZColumn<T>&
             num.x += g * xi.x;
             num.y += g * xi.y;
         }
-        v = mkc<T>(num.x * inv, num.y * inv);
+        v = mkc<T>(num.x / denom, num.y / denom);
     } else {
         T ca, cb, cg;
         prop_coef<PROP, T>(dopx, a.dt, deps, ca, cb, cg);
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     __syncthreads();
     // a ky-slab of a larger field: wavenumbers, the k = 0 mode and the noise keys of the field
     const int kyg = ky + a.ky0;
-    const T k1 = kwave_ck<T>(kyg, a.nyg, a.cky);
+    const T k1 = a.cky.at(kyg, a.nyg);
     const T deps = T(1) + a.C - a.eps;
     float mc = 0.f;
     T bad = T(0);
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
         const cx<T> psi_a = CARRY ? *g : zero, psi_b = CARRY && both ? g[tile.second] : zero;
         const el<T> psi = CARRY ? Elem<T>::pack(psi_a, psi_b) : buf[lay.at(i, at)];
         const el<T> nl = *slot;
-        const T kk2 = kwave_ck<T>(kz, n, a.ckz);
+        const T kk2 = a.ckz.at(kz, n);
         auto update = [&](cx<T> ps, cx<T> f, const ZColumn<T>& col) {
             if (!CARRY && conserved && col.kx == 0 && kyg == 0 && kz == 0)
                 ps = mkc<T>((T)k0[blockIdx.z].x, (T)k0[blockIdx.z].y);
@@ -219,10 +223,10 @@ __global__ void __launch_bounds__(256) k_zflat(cx<T>* A, const cx<T>* B, int nx,
     bool bad = false;
     if (m < nxh * ny) {
         const int ky = fdiv(m, by_nxh), kx = m - ky * nxh, kyg = ky + a.ky0;
-        const ZColumn<T> col(kx, nx, kwave_ck<T>(kyg, a.nyg, a.cky), a);
+        const ZColumn<T> col(kx, nx, a.cky.at(kyg, a.nyg), a);
         cx<T> psi = A[m];
         if (kx == 0 && kyg == 0 && a.prop != kPropRelax && a.prop != kPropRelaxExp) psi = mkc<T>((T)k0->x, (T)k0->y);
-        const cx<T> v = zmode<T>(a.prop, psi, B[m], col, kyg, 0, kwave_ck<T>(0, 1, a.ckz), nx, 1, T(1) + a.C - a.eps, a, mc);
+        const cx<T> v = zmode<T>(a.prop, psi, B[m], col, kyg, 0, a.ckz.at(0, 1), nx, 1, T(1) + a.C - a.eps, a, mc);
         bad = !isfinite(v.x) || !isfinite(v.y);
         A[m] = v;
     }
@@ -249,8 +253,8 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
     const int ny = flat ? 1 : c->ny, tile = ap.w << ap.lg;
     const double tp = 6.283185307179586232;
     dim3 grid((c->nxh + tile - 1) / tile, ny, c->batch);
-    ZArgsT<T> t{(T)a.dt, (T)a.eps, (T)a.C, (T)a.namp_eff, (T)(tp / a.lx), flat ? T(0) : (T)(tp / a.ly),
-                (T)(tp / (flat ? a.ly : a.lz)), a.seed, a.counter, a.dev_counter, a.use_noise, a.final_step, a.prop,
+    ZArgsT<T> t{(T)a.dt, (T)a.eps, (T)a.C, (T)a.namp_eff, Wave<T>(tp / a.lx), Wave<T>(flat ? 0.0 : tp / a.ly),
+                Wave<T>(tp / (flat ? a.ly : a.lz)), a.seed, a.counter, a.dev_counter, a.use_noise, a.final_step, a.prop,
                 a.maxc, a.margs, a.ky0, a.ny_global > 0 ? a.ny_global : ny};
     if (!flat && !carry && c->nz == 1 && c->batch == 1) {
         const int modes = c->nxh * c->ny;
