@@ -21,7 +21,7 @@ namespace {
 
 constexpr int kNQ = 9 + 13 + 17;         // q_lm, l = 4, 6, 8, m = -l..l
 constexpr int kW4 = 61, kW6 = 127;       // (l l l; m1 m2 m3) with m1 + m2 + m3 = 0
-__constant__ double c_nlm[3][9];         // normalisation of P_l^m, l = 4, 6, 8, m = 0..l
+__constant__ double c_nlm[3][9];         // normalisation of (l - m)! P_l^m, l = 4, 6, 8, m = 0..l
 __constant__ double c_w4[kW4];
 __constant__ int c_w4m[kW4][2];
 __constant__ double c_w6[kW6];
@@ -321,14 +321,12 @@ __global__ void __launch_bounds__(128) k_qlm(const double* __restrict__ pos, con
     const int* list = nbr + (i < P ? nb_off[i] : 0);
     double xi = 0.0, yi = 0.0, zi = 0.0;
     if (i < P) { xi = pos[3 * i]; yi = pos[3 * i + 1]; zi = pos[3 * i + 2]; }
-    // (l + m - 1) / (l - m) and (2 l - 1) / (l - m) of the recurrence
-    double ra[9], rb[9];
+    // Q_l = (l - m)! P_l^m: Q_l = (2 l - 1) x Q_{l-1} - (l + m - 1)(l - m - 1) Q_{l-2}, whole
+    // numbers where the recurrence of P_l^m divides by l - m (multiplying by its rounded reciprocal
+    // instead costs digits)
+    double rb[9];
 #pragma unroll
-    for (int l = 1; l <= 8; ++l) {
-        const double inv = l > m ? 1.0 / (double)(l - m) : 0.0;
-        ra[l] = (double)(2 * l - 1) * inv;
-        rb[l] = (double)(l + m - 1) * inv;
-    }
+    for (int l = 1; l <= 8; ++l) rb[l] = l > m ? (double)((l + m - 1) * (l - m - 1)) : 0.0;
     const double n4 = c_nlm[0][m], n6 = c_nlm[1][m], n8 = c_nlm[2][m];
     double2 p4 = make_double2(0.0, 0.0), p6 = p4, p8 = p4, s4 = p4, s6 = p4, s8 = p4;  // sums for +m, -m
     for (int a0 = 0; a0 < most; a0 += 9) {
@@ -361,7 +359,7 @@ __global__ void __launch_bounds__(128) k_qlm(const double* __restrict__ pos, con
             double p0 = 0.0, p1 = m == 0 ? 1.0 : 0.0, v4 = 0.0, v6 = 0.0, v8 = 0.0;
 #pragma unroll
             for (int l = 1; l <= 8; ++l) {
-                const double p2 = l == m ? pmm : xb * ra[l] * p1 - rb[l] * p0;  // (0 while l < m)
+                const double p2 = l == m ? pmm : (double)(2 * l - 1) * xb * p1 - rb[l] * p0;  // (0 while l < m)
                 p0 = p1;
                 p1 = p2;
                 if (l == 4) v4 = n4 * p2;
@@ -570,7 +568,7 @@ cudaError_t upload_tables() {
     const int ls[3] = {4, 6, 8};
     for (int li = 0; li < 3; ++li)
         for (int m = 0; m <= ls[li]; ++m)
-            nlm[li][m] = std::sqrt((2 * ls[li] + 1) / (4.0 * kPi) * fact(ls[li] - m) / fact(ls[li] + m));
+            nlm[li][m] = std::sqrt((2 * ls[li] + 1) / (4.0 * kPi) / (fact(ls[li] - m) * fact(ls[li] + m)));
     std::vector<double> w4, w6;
     std::vector<int> m4, m6;
     for (int a = -4; a <= 4; ++a)
