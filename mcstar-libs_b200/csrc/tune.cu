@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <map>
@@ -53,21 +54,31 @@ std::string options_json(const pfc_options& o, double ms) {
     return s.str();
 }
 
-// The cache file: {"pfc_tune": 1, "entries": {"<key>": {...}, ...}} with one entry per
-// line, as options_json writes them.  Returns the entries as key -> object text.
+// The cache file: {"pfc_tune": <revision>, "entries": {"<key>": {...}, ...}} with one entry per
+// line, as options_json writes them.  Returns the entries as key -> object text.  The revision
+// counts changes of what the options mean (2: radix_order and tile_shift name the in-place
+// engine's radices and tiles): entries of another were measured on other kernels, and none is returned.
+constexpr int kTuneRevision = 2;
+
 std::map<std::string, std::string> read_cache(const char* path) {
     std::map<std::string, std::string> out;
     std::ifstream f(path);
     if (!f) return out;
     std::string line;
+    int revision = 0;
     while (std::getline(f, line)) {
         const size_t q0 = line.find('"');
         const size_t q1 = q0 == std::string::npos ? q0 : line.find('"', q0 + 1);
-        const size_t b0 = q1 == std::string::npos ? q1 : line.find('{', q1);
-        const size_t b1 = line.rfind('}');
-        if (b0 == std::string::npos || b1 == std::string::npos || b1 < b0) continue;
+        if (q1 == std::string::npos) continue;
         const std::string key = line.substr(q0 + 1, q1 - q0 - 1);
-        if (key == "pfc_tune" || key == "entries") continue;
+        if (key == "pfc_tune") {
+            const size_t colon = line.find(':', q1);
+            revision = colon == std::string::npos ? 0 : std::atoi(line.c_str() + colon + 1);
+            continue;
+        }
+        const size_t b0 = line.find('{', q1), b1 = line.rfind('}');
+        if (b0 == std::string::npos || b1 == std::string::npos || b1 < b0) continue;
+        if (key == "entries" || revision != kTuneRevision) continue;
         out[key] = line.substr(b0, b1 - b0 + 1);
     }
     return out;
@@ -78,7 +89,7 @@ bool write_cache(const char* path, const std::map<std::string, std::string>& ent
     {
         std::ofstream f(tmp);
         if (!f) return false;
-        f << "{\"pfc_tune\": 1, \"entries\": {\n";
+        f << "{\"pfc_tune\": " << kTuneRevision << ", \"entries\": {\n";
         size_t i = 0;
         for (const auto& kv : entries)
             f << "  \"" << kv.first << "\": " << kv.second << (++i < entries.size() ? ",\n" : "\n");
