@@ -252,8 +252,10 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
     const AxisPlan& ap = flat ? c->py2 : carry ? c->pzprop : c->pz2;
     const int ny = flat ? 1 : c->ny, tile = ap.w << ap.lg;
     const double tp = 6.283185307179586232;
+    // (kz = 0 of a 2D field: zero, or not a number for an lz that gives none)
+    const double kz0 = flat ? (double)(T(0) * (T)tp / (T)a.lz) : 0.0;
     dim3 grid((c->nxh + tile - 1) / tile, ny, c->batch);
-    ZArgsT<T> t{(T)a.dt, (T)a.eps, (T)a.C, (T)a.namp_eff, Wave<T>(tp / a.lx), Wave<T>(flat ? 0.0 : tp / a.ly),
+    ZArgsT<T> t{(T)a.dt, (T)a.eps, (T)a.C, (T)a.namp_eff, Wave<T>(tp / a.lx + kz0), Wave<T>(flat ? 0.0 : tp / a.ly),
                 Wave<T>(tp / (flat ? a.ly : a.lz)), a.seed, a.counter, a.dev_counter, a.use_noise, a.final_step, a.prop,
                 a.maxc, a.margs, a.ky0, a.ny_global > 0 ? a.ny_global : ny};
     if (!flat && !carry && c->nz == 1 && c->batch == 1) {
