@@ -194,7 +194,7 @@ __device__ __forceinline__ double get_diff(double x1, double x2, double w) {
 struct Within {
     double rlim, lo, hi;
     explicit Within(double r) : rlim(r), lo(r * r * (1.0 - 1e-12)), hi(r * r * (1.0 + 1e-12)) {
-        if (!(r > 1e-100)) {  // (no square to compare with: always the root)
+        if (!(r > 1e-100 && r < 1e150)) {  // (no square to compare with: always the root)
             lo = -1.0;
             hi = INFINITY;
         }
