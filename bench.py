@@ -153,7 +153,7 @@ def kernel_table(prof, S, steps, x_kernel=0, y_kernel=0):
     elif prof["xy_mode"] == 1:
         add("k_plane_xy", 1, 2.0 * S)
     else:
-        add("k_cols+k_xpass+k_cols", 1, 6.0 * S)
+        add("k_cols+k_xpass or k_rows+k_cols", 1, 6.0 * S)  # (the x pass by the row length)
     if prof["z_mode"] in (2, 4, 5):
         # psi^ and B read, psi^' and A' written; the last step of a run writes psi^' only
         name = {4: "k_zbulk", 2: "k_zcarry", 5: "k_zprop (psi^ carried)"}[prof["z_mode"]]

@@ -200,8 +200,8 @@ cudaError_t step_entry(pfc_ctx* ctx, void* kpsi) {
             if (!e) e = launch_zfft(ctx, 1, kpsi, ctx->work, 1.0 / ctx->nz, kLayZ << 2, 0, -1, ctx->work2);
             return e;
         });
-    if (ctx->nz == 1)  // 2D: A = IFFT_y(psi^)/ny, psi^ carried in its buffer
-        return traced(ctx, 0, 1, [&] { return launch_cols(ctx, 1, 1, kpsi, ctx->work, 1.0 / ctx->ny); });
+    if (ctx->nz == 1)  // 2D: A = IFFT_y(psi^) (the x pass scales), psi^ carried in its buffer
+        return traced(ctx, 0, 1, [&] { return launch_cols(ctx, 1, 1, kpsi, ctx->work, 1.0); });
     if (ctx->z_carry && !ctx->fused_z)  // the inverse transform of the z pass itself; psi^ keeps its k = 0 mode
         return traced(ctx, 0, 1, [&] { return launch_cols(ctx, 2, 1, kpsi, ctx->work2, 1.0 / ctx->nz); });
     return traced(ctx, 0, 2, [&] {
@@ -235,10 +235,8 @@ cudaError_t step_xy(pfc_ctx* ctx, void* kpsi, const pfc_step_params* p, bool las
     const double mul = 1.0 / ((double)ctx->nx * (double)ctx->ny);
     if (ctx->nz == 1)  // 2D: the rows of A in place (the y transforms are the update pass's)
         return traced(ctx, 1, 1, [&] {
-            // A holds the factor 1/ny, rounded: the rest, so that the product is off by one rounding
-            const double inv = 1.0 / ctx->ny, rest = mul / (ctx->dtype == PFC_F64 ? inv : (double)(float)inv);
-            if (ctx->xy_mode == 2) return launch_xpass(ctx, B, nullptr, rest, p->C, p->mu, 1);
-            return launch_rows_nonlin(ctx, B, rest, p->C, p->mu);
+            if (ctx->xy_mode == 2) return launch_xpass(ctx, B, nullptr, mul, p->C, p->mu, 1);
+            return launch_rows_nonlin(ctx, B, mul, p->C, p->mu);
         });
     if (ctx->tiled) {
         void* R = row_field(ctx, kpsi);

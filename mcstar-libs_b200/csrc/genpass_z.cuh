@@ -113,7 +113,7 @@ __device__ __forceinline__ cx<T> zmode(int prop, A&&... args) {
 // A tile of kx columns (2^lg elements of n modes, at one ky) per CTA, over the reference layout.
 // CARRY true: psi^ itself is carried in A; N^ = FFT(B), the update writes psi^' over psi^, and
 // A' = IFFT(psi^')/n goes to anext (which may be B: a CTA reads its columns before it writes
-// them; not written on the final step).  CARRY false (ky-slabs, and schedules that ask for
+// them; not written on the final step; in a 2D field without the 1/n, which its x pass applies).  CARRY false (ky-slabs, and schedules that ask for
 // it): A = IFFT(psi^)/n is carried; psi^ = FFT(A), N^ = FFT(B), the update, A' over A (psi^'
 // on the final step), the k = 0 mode from its FP64 slot.  The N^ lines (and with CARRY false
 // the psi^ lines beside them) stay in shared memory, digit-reversed, between the transforms.
@@ -121,7 +121,7 @@ template <typename T, bool CARRY>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_zprop(cx<T>* A, const cx<T>* B, int nx, int ny, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
             const int* __restrict__ tab, int lg, int w, ZArgsT<T> a, const double2* k0, int* flag, int64_t ms,
-            cx<T>* anext, int lead) {
+            cx<T>* anext, double rn, int lead) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
     chain_start(lead);
@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     stages_back<T, 1>(buf, p, lay, tw);
     chain_start();
     cx<T>* dst = CARRY ? anext + base : A;
-    // (the entry transform's scale, so that a resumed run repeats the bits)
-    const typename Elem<T>::real scale = Elem<T>::bc(1.0 / (double)n);
+    // (rn: the entry transform's scale, so that a resumed run repeats the bits)
+    const typename Elem<T>::real scale = Elem<T>::bc(rn);
     stage_out<T, 1>(buf, p, lay, tw, [&](int i, int j, int m) {
         const int c = i & tmask;
         const bool ok0 = i >= nl0 && tile.ok(c, 0), ok1 = i >= nl0 && tile.ok(c, 1);
@@ -267,7 +267,7 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
     auto k = carry ? k_zprop<T, true> : k_zprop<T, false>;
     return chain_launch(c, k, grid, ap.threads, carry ? ap.smem : 2 * ap.smem, (cx<T>*)A, (const cx<T>*)B, c->nx, ny,
                         ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, ap.w, t, c->k0, c->flag, c->mstride,
-                        (cx<T>*)anext);
+                        (cx<T>*)anext, flat ? 1.0 : 1.0 / (double)ap.plan.n);
 }
 
 }  // namespace pfc
