@@ -87,7 +87,8 @@ pfc_status  pfc_destroy(pfc_ctx* ctx);
  * the current device -- a coordinate search, one option at a time from the library's
  * choice -- and returns the fastest in *best (and its time per step in *ms_per_step, may
  * be NULL).  With a cache_path, results are kept in that JSON file keyed by shape,
- * precision and device, and a cached entry is returned without timing.  Tuning creates
+ * precision and device, and a cached entry is returned without timing (one of a file written
+ * when the options meant something else is timed again).  Tuning creates
  * and destroys contexts and allocates device memory (setup time, not the step). */
 typedef struct pfc_options {
     int z_carry;
