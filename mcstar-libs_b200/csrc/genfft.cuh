@@ -37,6 +37,7 @@ struct GStage {
 };
 struct GPlan {
     int n, nst;
+    int odd;      // 1: a radix of 7, or of 11 to 31
     int np;       // shared-memory elements of a line (padding included)
     int rl, pad;  // last radix; 1 where it is even (padded)
     int kstep;    // n / rl: distance of the frequencies of a last-stage butterfly
@@ -330,8 +331,11 @@ template <typename T, int DIR> struct EDft<T, DIR, 7> : DftOdd<T, DIR, 7> {};
 template <typename T, int DIR> struct EDft<T, DIR, 9> : DftSq<T, DIR, 3> {};
 template <typename T, int DIR> struct EDft<T, DIR, 10> : DftPfa<T, DIR, 5, 2> {};
 
-// f(std::integral_constant<int, R>) for a stage's radix; 0 stands for a prime radix from 11 up
-template <class F> __device__ __forceinline__ void by_radix(int R, F&& f) {
+// f(std::integral_constant<int, R>) for a stage's radix; 0 stands for a prime radix from 11 up.  ODD:
+// the plan may have radices 7 and 11 to 31.  Those are instantiated apart: in one body with the others
+// they take registers from all (192^3 FP64 204.6 us per step with all radices in one body, 201.3 so;
+// 240 x 200 x 180 FP32 with noise 168.4 and 165.9).
+template <bool ODD, class F> __device__ __forceinline__ void by_radix(int R, F&& f) {
     switch (R) {
         case 1: f(std::integral_constant<int, 1>{}); break;
         case 2: f(std::integral_constant<int, 2>{}); break;
@@ -339,11 +343,15 @@ template <class F> __device__ __forceinline__ void by_radix(int R, F&& f) {
         case 4: f(std::integral_constant<int, 4>{}); break;
         case 5: f(std::integral_constant<int, 5>{}); break;
         case 6: f(std::integral_constant<int, 6>{}); break;
-        case 7: f(std::integral_constant<int, 7>{}); break;
         case 8: f(std::integral_constant<int, 8>{}); break;
         case 9: f(std::integral_constant<int, 9>{}); break;
         case 10: f(std::integral_constant<int, 10>{}); break;
-        default: f(std::integral_constant<int, 0>{}); break;
+        default:
+            if constexpr (ODD) {
+                if (R == 7) f(std::integral_constant<int, 7>{});
+                else f(std::integral_constant<int, 0>{});
+            }
+            break;
     }
 }
 
@@ -429,7 +437,8 @@ __device__ __forceinline__ int gpad(const GPlan& p, int i) { return p.pad ? i + 
 
 // How a pass lays its lines out: element position a of line i at at(i, a), and butterfly
 // e of a stage with nb butterflies per line -> (line, index).
-struct ColLines {  // lines interleaved: consecutive threads move one element of each of 2^lg lines (FP32: pairs)
+template <bool ODD> struct ColLines {  // lines interleaved: consecutive threads move one element of each of 2^lg lines (FP32: pairs)
+    static constexpr bool odd = ODD;
     int lg;
     __device__ __forceinline__ int count(int nb) const { return nb << lg; }
     __device__ __forceinline__ void split(int e, int, FastDiv, int& i, int& q) const {
@@ -439,7 +448,8 @@ struct ColLines {  // lines interleaved: consecutive threads move one element of
     __device__ __forceinline__ int at(int i, int a) const { return (a << lg) + i; }
     __device__ __forceinline__ int step(int a) const { return a << lg; }
 };
-struct RowLines {  // whole lines one after the other: consecutive threads move consecutive elements
+template <bool ODD> struct RowLines {  // whole lines one after the other: consecutive threads move consecutive elements
+    static constexpr bool odd = ODD;
     int lines, np;
     __device__ __forceinline__ int count(int nb) const { return lines * nb; }
     __device__ __forceinline__ void split(int e, int nb, FastDiv by_nb, int& i, int& q) const {
@@ -456,7 +466,7 @@ __device__ __forceinline__ void stage_inplace(el<T>* buf, const GPlan& p, int si
                                               const el<T>* __restrict__ tw) {
     const GStage& s = p.st[si];
     const int total = lay.count(s.nb), step = lay.step(s.ms);
-    by_radix(s.R, [&](auto RC) {
+    by_radix<L::odd>(s.R, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         for (int e = threadIdx.x; e < total; e += blockDim.x) {
             int i, q;
@@ -476,7 +486,7 @@ __device__ __forceinline__ void stage_first(el<T>* buf, const GPlan& p, const L&
                                             In in) {
     const GStage& s = p.st[0];
     const int total = lay.count(s.m), step = lay.step(s.ms);
-    by_radix(s.R, [&](auto RC) {
+    by_radix<L::odd>(s.R, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         for (int e = threadIdx.x; e < total; e += blockDim.x) {
             int i, j;
@@ -495,7 +505,7 @@ __device__ __forceinline__ void stage_last(el<T>* buf, const GPlan& p, const L& 
                                            const int* __restrict__ rev, Out out) {
     const GStage& s = p.st[p.nst - 1];
     const int total = lay.count(p.kstep), step = lay.step(1);
-    by_radix(s.R, [&](auto RC) {
+    by_radix<L::odd>(s.R, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         if constexpr (R > 0) {  // (the host appends a stage of radix 1 to a prime radix)
             for (int e = threadIdx.x; e < total; e += blockDim.x) {
@@ -516,7 +526,7 @@ __device__ __forceinline__ void stage_in(el<T>* buf, const GPlan& p, const L& la
                                          const int* __restrict__ rev, In in) {
     const GStage& s = p.st[p.nst - 1];
     const int total = lay.count(p.kstep), step = lay.step(1);
-    by_radix(s.R, [&](auto RC) {
+    by_radix<L::odd>(s.R, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         if constexpr (R > 0) {
             for (int e = threadIdx.x; e < total; e += blockDim.x) {
@@ -537,7 +547,7 @@ __device__ __forceinline__ void stage_out(el<T>* buf, const GPlan& p, const L& l
                                           Out out) {
     const GStage& s = p.st[0];
     const int total = lay.count(s.m), step = lay.step(s.ms);
-    by_radix(s.R, [&](auto RC) {
+    by_radix<L::odd>(s.R, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         for (int e = threadIdx.x; e < total; e += blockDim.x) {
             int i, j;

@@ -14,7 +14,7 @@ namespace {
 // transforms run down from natural order, inverse ones up to it: the inverse is then, bit
 // for bit, the one of the stepper's z pass (k_zprop).
 // ---------------------------------------------------------------------------------
-template <typename T, int DIR>
+template <typename T, int DIR, bool ODD>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_cols(const cx<T>* in, cx<T>* out, int ni, int64_t es, int64_t os, const __grid_constant__ GPlan p,
            const el<T>* __restrict__ tw, const int* __restrict__ tab, int lg, int w, double scale,
@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     el<T>* buf = reinterpret_cast<el<T>*>(smem_raw);
     chain_start(lead);
     chain_wait();
-    const ColLines lay{lg};
+    const ColLines<ODD> lay{lg};
     const ColTile<T> tile{lg, w, ni};
     const int64_t base = (int64_t)blockIdx.y * os + tile.i0 + blockIdx.z * ms;  // grid z: fields of a batch
     in += base;
@@ -91,7 +91,7 @@ __device__ __forceinline__ R cubic(R v, R mul, R nC, R nmu) {  // nC = -C, nmu =
 // the engine: whole rows (W = 1; FP32: each twice) or pairs of rows (FP32, W = 2).  The transforms leave
 // frequencies (or cells) digit-reversed; the R2C merge and the C2R output read them back in
 // natural order through the position table, so that global accesses stay contiguous.
-template <typename T, int MODE>
+template <typename T, int MODE, bool ODD>
 __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
     k_rows(const void* in, void* out, int nrows, int nx, const __grid_constant__ GPlan p,
            const el<T>* __restrict__ tw, const int* __restrict__ tab, const el<T>* __restrict__ post, int rpc,
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
     if (Elem<T>::lines == 1) W = 1;
     const int row0 = blockIdx.x * rpc * W;
     const int nr = min(rpc * W, nrows - row0), nl = W > 1 ? (nr + 1) / 2 : nr;
-    const RowLines lay{nl, p.np};
+    const RowLines<ODD> lay{nl, p.np};
     const int L = p.n, nxh = nx / 2 + 1;
     const bool even = (nx & 1) == 0;
     const int* pos = tab + p.pos;
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kGenThreads, kGenCtas<T>)
         const auto bmul = Elem<T>::bc(mul), nC = Elem<T>::bc(-C), nmu = Elem<T>::bc(-mu);
         const GStage& s = p.st[p.nst - 1];
         const int total = lay.count(p.kstep);
-        by_radix(s.R, [&](auto RC) {
+        by_radix<ODD>(s.R, [&](auto RC) {
             constexpr int R = decltype(RC)::value;
             if constexpr (R > 0) {
                 for (int e = threadIdx.x; e < total; e += blockDim.x) {
@@ -230,7 +230,7 @@ template <class F> __device__ __forceinline__ void by_pair_radix(int R, F&& f) {
 // 80 registers (three CTAs per SM): at 64 the radix-5 pair spills.  A step against the general kernel,
 // us: 240x200x180 FP32 149.0 -> 144.2, 1000x900 FP64 39.6 -> 35.1, 90x80x100 FP32
 // 37.5 -> 33.7, 2400x2000 FP32 95.8 -> 90.2.
-template <typename T>
+template <typename T, bool ODD>
 __global__ void __launch_bounds__(kGenThreads, 3)
     k_xpass(cx<T>* field, int nrows, int nxh, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
             const el<T>* __restrict__ post, int rpc, int W, FastDiv by_half, double mul, double C, double mu,
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kGenThreads, 3)
     if (E::lines == 1) W = 1;
     const int row0 = blockIdx.x * rpc * W;
     const int nr = min(rpc * W, nrows - row0), nl = W > 1 ? (nr + 1) / 2 : nr;
-    const RowLines lay{nl, p.np};
+    const RowLines<ODD> lay{nl, p.np};
     const int L = p.n;
     const GStage& s0 = p.st[0];
     const int m = s0.m, half = m / 2 + 1, total = nl * half;
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kGenThreads, 3)
         const auto bmul = E::bc(mul), nC = E::bc(-C), nmu = E::bc(-mu);
         const GStage& s = p.st[p.nst - 1];
         const int count = lay.count(p.kstep);
-        by_radix(s.R, [&](auto RC) {
+        by_radix<ODD>(s.R, [&](auto RC) {
             constexpr int R = decltype(RC)::value;
             if constexpr (R > 0) {
                 for (int e = threadIdx.x; e < count; e += blockDim.x) {
@@ -359,16 +359,20 @@ __global__ void __launch_bounds__(kGenThreads, 3)
 
 }  // namespace
 
-template <typename T> cudaError_t gen_attrs() {
+template <typename T, bool ODD> cudaError_t gen_attrs_of() {
     const int m = (int)kMaxDynSmem;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(k_cols<T, -1>, attr, m);
-    if (!e) e = cudaFuncSetAttribute(k_cols<T, 1>, attr, m);
-    if (!e) e = cudaFuncSetAttribute(k_rows<T, kR2C>, attr, m);
-    if (!e) e = cudaFuncSetAttribute(k_rows<T, kC2R>, attr, m);
-    if (!e) e = cudaFuncSetAttribute(k_rows<T, kNonlin>, attr, m);
-    if (!e) e = cudaFuncSetAttribute(k_xpass<T>, attr, m);
+    cudaError_t e = cudaFuncSetAttribute(k_cols<T, -1, ODD>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_cols<T, 1, ODD>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_rows<T, kR2C, ODD>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_rows<T, kC2R, ODD>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_rows<T, kNonlin, ODD>, attr, m);
+    if (!e) e = cudaFuncSetAttribute(k_xpass<T, ODD>, attr, m);
     return e;
+}
+template <typename T> cudaError_t gen_attrs() {
+    const cudaError_t e = gen_attrs_of<T, false>();
+    return e ? e : gen_attrs_of<T, true>();
 }
 
 template <typename T>
@@ -382,7 +386,8 @@ cudaError_t gen_cols(const pfc_ctx* c, int axis, int dir, const void* in, void* 
     else { es = (int64_t)c->ny * c->nxh; os = c->nxh; no = c->ny; }
     const int tile = ap.w << ap.lg;
     dim3 grid((c->nxh + tile - 1) / tile, no, c->batch);
-    auto k = dir < 0 ? k_cols<T, -1> : k_cols<T, 1>;
+    auto k = ap.plan.odd ? (dir < 0 ? k_cols<T, -1, true> : k_cols<T, 1, true>)
+                         : (dir < 0 ? k_cols<T, -1, false> : k_cols<T, 1, false>);
     return chain_launch(c, k, grid, ap.threads, ap.smem, (const cx<T>*)in, (cx<T>*)out, c->nxh, es, os, ap.plan,
                         (const el<T>*)c->gtw, c->fft_tab, ap.lg, ap.w, scale, c->mstride);
 }
@@ -394,7 +399,8 @@ cudaError_t gen_rows(const pfc_ctx* c, int mode, const void* in, void* out, doub
         const AxisPlan& ap = c->px2;
         const el<T>* tw = (const el<T>*)c->gtw;
         const int rows = ap.lines * ap.w;
-        return chain_launch(c, k_xpass<T>, dim3((nrows + rows - 1) / rows, 1, c->batch), ap.threads, ap.smem,
+        auto k = ap.plan.odd ? k_xpass<T, true> : k_xpass<T, false>;
+        return chain_launch(c, k, dim3((nrows + rows - 1) / rows, 1, c->batch), ap.threads, ap.smem,
                             (cx<T>*)out, nrows, c->nxh, ap.plan, tw, tw + c->post_off, ap.lines, ap.w,
                             make_fastdiv(ap.plan.st[0].m / 2 + 1), mul, C, mu, c->mstride);
     }
@@ -403,7 +409,8 @@ cudaError_t gen_rows(const pfc_ctx* c, int mode, const void* in, void* out, doub
     const int rows = ap.lines * ap.w;
     // (the plain transforms run on one field; the x pass on all fields of a batch)
     dim3 grid((nrows + rows - 1) / rows, 1, mode == kNonlin ? c->batch : 1);
-    auto k = mode == kR2C ? k_rows<T, kR2C> : mode == kC2R ? k_rows<T, kC2R> : k_rows<T, kNonlin>;
+    auto k = ap.plan.odd ? (mode == kR2C ? k_rows<T, kR2C, true> : mode == kC2R ? k_rows<T, kC2R, true> : k_rows<T, kNonlin, true>)
+                         : (mode == kR2C ? k_rows<T, kR2C, false> : mode == kC2R ? k_rows<T, kC2R, false> : k_rows<T, kNonlin, false>);
     return chain_launch(c, k, grid, ap.threads, ap.smem, in, out, nrows, c->nx, ap.plan, tw, c->fft_tab,
                         tw + c->post_off, ap.lines, ap.w, mul, C, mu, c->mstride, make_fastdiv(c->nxh));
 }

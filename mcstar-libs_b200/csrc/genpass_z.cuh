@@ -117,7 +117,7 @@ __device__ __forceinline__ cx<T> zmode(int prop, A&&... args) {
 // it): A = IFFT(psi^)/n is carried; psi^ = FFT(A), N^ = FFT(B), the update, A' over A (psi^'
 // on the final step), the k = 0 mode from its FP64 slot.  The N^ lines (and with CARRY false
 // the psi^ lines beside them) stay in shared memory, digit-reversed, between the transforms.
-template <typename T, bool CARRY>
+template <typename T, bool CARRY, bool ODD>
 __global__ void __launch_bounds__(kColThreads<T>, 1)
     k_zprop(cx<T>* A, const cx<T>* B, int nx, int ny, const __grid_constant__ GPlan p, const el<T>* __restrict__ tw,
             const int* __restrict__ tab, int lg, int w, ZArgsT<T> a, const double2* k0, int* flag, int64_t ms,
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kColThreads<T>, 1)
     B += base;
     // the lines in shared memory: the tile's N^ lines, after its psi^ lines when they are
     // transformed too
-    const ColLines lay{CARRY ? lg : lg + 1};
+    const ColLines<ODD> lay{CARRY ? lg : lg + 1};
     const int tmask = (1 << lg) - 1, nl0 = CARRY ? 0 : 1 << lg;
     stage_first<T, -1>(buf, p, lay, tw, [&](int i, int j, int m) {
         const int c = i & tmask;
@@ -238,8 +238,10 @@ __global__ void __launch_bounds__(256) k_zflat(cx<T>* A, const cx<T>* B, int nx,
 
 template <typename T> cudaError_t gen_zattrs() {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(k_zprop<T, false>, attr, (int)kMaxDynSmem);
-    if (!e) e = cudaFuncSetAttribute(k_zprop<T, true>, attr, (int)kMaxDynSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_zprop<T, false, false>, attr, (int)kMaxDynSmem);
+    if (!e) e = cudaFuncSetAttribute(k_zprop<T, true, false>, attr, (int)kMaxDynSmem);
+    if (!e) e = cudaFuncSetAttribute(k_zprop<T, false, true>, attr, (int)kMaxDynSmem);
+    if (!e) e = cudaFuncSetAttribute(k_zprop<T, true, true>, attr, (int)kMaxDynSmem);
     return e;
 }
 
@@ -264,7 +266,8 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
                                                                make_fastdiv(c->nxh), t, c->k0, c->flag);
         return cudaGetLastError();
     }
-    auto k = carry ? k_zprop<T, true> : k_zprop<T, false>;
+    auto k = ap.plan.odd ? (carry ? k_zprop<T, true, true> : k_zprop<T, false, true>)
+                         : (carry ? k_zprop<T, true, false> : k_zprop<T, false, false>);
     return chain_launch(c, k, grid, ap.threads, carry ? ap.smem : 2 * ap.smem, (cx<T>*)A, (const cx<T>*)B, c->nx, ny,
                         ap.plan, (const el<T>*)c->gtw, c->fft_tab, ap.lg, ap.w, t, c->k0, c->flag, c->mstride,
                         (cx<T>*)anext, flat ? 1.0 : 1.0 / (double)ap.plan.n);

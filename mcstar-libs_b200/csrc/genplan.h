@@ -94,6 +94,7 @@ inline bool make_plan(int n, GPlan& p, std::vector<std::complex<double>>& tab, s
     for (int s = 0; s < p.nst; ++s) {
         GStage& g = p.st[s];
         g.R = rs[s];
+        if (g.R == 7 || g.R > 10) p.odd = 1;
         g.m = M / g.R;
         g.nb = n / g.R;
         p.nbmax = std::max(p.nbmax, g.nb);
