@@ -157,7 +157,7 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
     // Rows: as many as fill those threads, by the butterflies of the largest prime radix where there is
     // one (a 209-point row in FP64 has 11 of radix 19, and by the stage with the most, the appended one of
     // radix 1, one row per CTA: 209x57x260 x pass 679 us, now 133).  With at most four CTAs per SM
-    // at least a thread for two points, for the loops over the row's modes (1024 x 240 FP32, two
+    // k_rows takes at least a thread for two points, for its loops over the row's modes (1024 x 240 FP32, two
     // rows: C2R rows 10.6 us at 64 threads, 9.0 at 256; 128 x 45 x 30, eight rows: R2C 5.1 at 64,
     // 4.4 at 256).
     const int W = c->dtype == PFC_F64 ? 1 : 2;  // lines of an element
@@ -191,8 +191,9 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
     columns(c->pzprop, c->ny, 1, true, o.tile_shift[3]);
     columns(c->pz2, c->ny, 2, true, o.tile_shift[3]);
     columns(c->py2, 1, 1, true, o.tile_shift[3]);
-    // work: the most items of a line in a stage; longest: in the stage that takes longest
-    auto rows = [&](AxisPlan& ap, int work, int longest) {
+    // work: the most items of a line in a stage; longest: in the stage that takes longest; merge: a pass
+    // with loops over the row's modes
+    auto rows = [&](AxisPlan& ap, int work, int longest, bool merge) {
         const int64_t nrows = (int64_t)c->ny * c->nz;
         int rpc = std::max(1, many / longest) * W;  // rows of a CTA
         auto bytes = [&] { return (size_t)(rpc / W) * ap.plan.np * 16; };
@@ -202,16 +203,16 @@ inline void plan_launches(pfc_ctx* c, const pfc_options& o, int batch, int sms) 
         ap.w = std::min(W, rpc);
         ap.lines = rpc / ap.w;
         int items = ap.lines * work;
-        if ((nrows + rpc - 1) / rpc * batch <= 4 * (int64_t)sms) items = std::max(items, ap.lines * ap.plan.n / 2);
+        if (merge && (nrows + rpc - 1) / rpc * batch <= 4 * (int64_t)sms) items = std::max(items, ap.lines * ap.plan.n / 2);
         ap.threads = std::min(kGenThreads, std::max(32, (items + 31) & ~31));
         ap.smem = (size_t)ap.lines * ap.plan.np * 16;
     };
-    rows(c->px, c->px.plan.nbmax, c->px.plan.nblong);
+    rows(c->px, c->px.plan.nbmax, c->px.plan.nblong, true);
     if (c->px2.plan.nst) {
         const GPlan& q = c->px2.plan;
         int work = q.st[0].m / 2 + 1;
         for (int i = 1; i < q.nst; ++i) work = std::max(work, q.st[i].nb);
-        rows(c->px2, work, work);
+        rows(c->px2, work, work, false);
     }
 }
 
