@@ -22,10 +22,10 @@ cudaError_t gen_zprop(const pfc_ctx* c, void* A, const void* B, const ZPropArgs&
 // temporaries).  They are latency-bound: at 128 registers and radices up to 16 the passes of
 // 240 x 200 x 180 FP32 took 0.025 / 0.049 / 0.088 ms (y, x, z) against 0.021 / 0.044 / 0.060.
 // The column passes may take the whole register file with one CTA: 1024 threads (FP64 768) of the
-// same registers, for fields with few tiles.  One body holds every radix (and k_zprop six
-// propagators), so the FP32 kernels spill at 64 registers: k_cols 32 and 140 bytes (inverse,
-// forward), k_rows 92 to 136, k_zprop 148 and 156; the direct DFT of a prime radix keeps its points in
-// local memory (a frame of 500 bytes).  k_xpass has 80 registers and does not spill.
+// same registers, for fields with few tiles.  One body holds the radices 1 to 6 and 8 to 10, so the FP32
+// kernels spill at 64 registers: k_cols 48 and 152 bytes (inverse, forward), k_rows 100 to 112,
+// k_zprop 120 to 176; k_xpass has 80 registers and does not spill.  The kernels of plans with radix 7 or
+// 11 to 31 are instantiated apart, with the points of a direct DFT in local memory.
 template <typename T> constexpr int kGenCtas = sizeof(T) == 8 ? 3 : 4;
 constexpr int kGenThreads = 256;
 template <typename T> constexpr int kColThreads = sizeof(T) == 8 ? 768 : 1024;
