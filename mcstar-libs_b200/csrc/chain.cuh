@@ -16,9 +16,9 @@
 // The launch gap of the small passes is what this removes: 1.6 us of a 5 us pass.  A next kernel that
 // starts while most of this one's work is still to come has its CTAs packed onto the few
 // multiprocessors with room left, and runs them there: with chain_start() at the beginning of every
-// CTA 192x128x32 FP32 with noise took 42.5 us per step, unchained 37.7, so 28.8; 64x64x64 15.2,
-// 20.1, 11.8; R2C of 1024^2 22.5, 17.4, 12.8.  In a grid of several waves the CTAs after the first
-// wave start it early, so that the next kernel fills the last wave's gaps (192x160x192 73 us per
+// CTA 192x128x32 FP32 with noise took 42.5 us per step, unchained 37.7, so 28.2; 64x64x64 15.2,
+// 20.1, 11.8; R2C of 1024^2 22.5, 17.4, 12.9.  In a grid of several waves the CTAs after the first
+// wave start it early, so that the next kernel fills the last wave's gaps (192x160x192 68 us per
 // step; with the late start alone 88).  Calls whose stream is being captured, and ensembles
 // (captured, several branches), launch plainly.
 #pragma once

@@ -382,7 +382,7 @@ __device__ __forceinline__ void gbfly(const GStage& s, const el<T>* __restrict__
         //   X[k], X[R-k] = x_0 + sum_r s_r cos(2 pi k r / R) +- DIR i sum_r d_r sin(2 pi k r / R),
         // two k at a time, and the loads of four pairs in flight.  (Loaded one by one, and multiplied
         // out as R^2 complex products, with the row plan of one row per CTA: a 247 x 105 x 182 FP64
-        // step 3836 us, now 375.)
+        // step 3860 us, now 367.)
         using RR = typename Elem<T>::real;
         el<T> v[kMaxOddRadix];
         const el<T>* wr = tw + s.rt;
